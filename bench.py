@@ -42,6 +42,7 @@ UNIT = "ct-mult+relin/s"
 # captures of the same kernels (dram__bytes_read.sum + dram__bytes_write.sum
 # of one 16-ciphertext launch); None where not captured.
 TRAFFIC_PER_CT = {
+    "ks32_rows": (103.5e6 + 4.1e6) / 16,    # k32_rows (writes still in L2)
     "ks_rows": (300.8e6 + 20.6e6) / 16,     # k4_ks_rows_warp
     "digit_cols": (12.7e6 + 169.2e6) / 16,  # k4_digit_cols_all
 }
@@ -50,13 +51,15 @@ TRAFFIC_PER_CT = {
 # the same ncu capture (sm__pipe_fmaheavy_cycles_active, one 16-ciphertext
 # launch).
 MULPIPE_BUSY = {
+    "ks32_rows": 0.590,   # k32_rows (of elapsed cycles)
     "ks_rows": 0.772,     # k4_ks_rows_warp
     "digit_cols": 0.761,  # k4_digit_cols_all
 }
 # Kernel scopes the library times (shg_profile_query) in one ct-mult+relin
-# step; the four-step key switch runs digit_cols + ks_rows, the unfused one
-# digit_ntt + ks_inner.
-SCOPES = ("tensor_intt", "digit_cols", "ks_rows", "digit_ntt", "ks_inner")
+# step; the key switch in three 32-bit primes runs the four ks32 kernels, the
+# four-step one digit_cols + ks_rows, the unfused one digit_ntt + ks_inner.
+SCOPES = ("tensor_intt", "ks32_digits", "ks32_rows", "ks32_crt", "ks32_out", "digit_cols",
+          "ks_rows", "digit_ntt", "ks_inner")
 
 
 def scope_model(name, n, L, k, cts):
@@ -66,11 +69,23 @@ def scope_model(name, n, L, k, cts):
     (c0, c1) and the plain c2 (7 polys); the digit kernels read c2 and write
     the k digit transforms; the inner-product kernels read the digit
     transforms, the base and write the result (k + 4 polys) plus the key once.
+    The ks32 kernels move 32-bit words: 3 per digit coefficient, 6 per limb's
+    sums and 6 per key coefficient.  Butterflies are the 64-bit ones (theirs
+    are 32-bit but for the reconstruction's column phase and the last rows).
     """
     poly = L * n * 8
     bfly_ntt = n // 2 * (n.bit_length() - 1)
     if name == "tensor_intt":
         return 7 * poly * cts, L * bfly_ntt * cts
+    words = n * 4
+    if name == "ks32_digits":
+        return (poly + 3 * k * words) * cts, 0
+    if name == "ks32_rows":
+        return (3 * k + 6 * L) * words * cts + 6 * k * L * words, 0
+    if name == "ks32_crt":
+        return (6 * L * words + 2 * poly) * cts, 2 * L * (n // 2) * (n.bit_length() - 1 - 7) * cts
+    if name == "ks32_out":
+        return 6 * poly * cts, 2 * L * (n // 2) * 7 * cts
     if name == "digit_ntt":
         return (1 + k) * poly * cts, k * L * bfly_ntt * cts
     if name == "digit_cols":
@@ -1958,7 +1973,7 @@ def main():
         "avg_launch_ms": tk["avg_launch_ms"],
         "multiply_pipe": {"busy_frac": MULPIPE_BUSY.get(top),
                           "source": "ncu sm__pipe_fmaheavy_cycles_active of one 16-ciphertext "
-                                    "launch: the kernel is bound by 64-bit integer multiply "
+                                    "launch: the kernel is bound by integer multiply "
                                     "throughput, not HBM"} if top in MULPIPE_BUSY else None,
         # The transforms are bound by 64-bit integer multiply issue, not HBM:
         # butterflies/s of the NTT-bearing kernels against the live probe.

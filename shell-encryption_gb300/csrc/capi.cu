@@ -206,6 +206,14 @@ struct shg_context {
   // Key-switch lanes of the host-buffer pipeline.
   cudaStream_t io_lanes[kMaxKsLanes] = {};
   std::mutex io_mu;
+  // Auxiliary primes of the 32-bit key switch (ks32.cu), made with the first
+  // key that uses them: [0] below 2^30, [1] below 2^28 (lazy), with twiddles
+  // [2][3][n] and one Crt32 per main limb.
+  struct Set32 {
+    shg::W32 w{};
+    uint2* d_tw = nullptr;
+    shg::Crt32* d_crt = nullptr;
+  } set32[2];
 
   CtxDev dev() const {
     return CtxDev{log_n, n, L, d_primes, d_tw_fwd, d_tw_inv, d_qmod, small_q, ntt4_min,
@@ -249,6 +257,8 @@ struct shg_key {
   int digit_flags = 0;  // shg::digit_flags(need_lift, largest log_b)
   int chunk = 1;       // digits per REDC for canonical digit transforms
   int chunk_lazy = 1;  // the same for lazily reduced ones (below 62 q)
+  shg::Ks32 ks32;           // the key in the 32-bit auxiliary primes, if it has that form
+  uint32_t* d_key32 = nullptr;
   size_t bytes = 0;
 };
 
@@ -291,6 +301,30 @@ int launch_status(const char* what) {
   cudaError_t e = cudaGetLastError();
   if (e != cudaSuccess) return cuda_fail(e, what);
   return SHG_OK;
+}
+
+// The key's 32-bit form if a key switch of `count` ciphertexts with this one
+// key should use it (ks32.cu), else an empty one.  Counted in 64-bit transforms
+// of n, it saves k L of them and costs 0.45 of one per 32-bit transform (3 k + 6 L)
+// and 2 L; two more launches need a saving of about 1.75 M coefficients (measured
+// break-even: n = 2^14, 6 limbs between 1 and 2 ciphertexts (49.7 / 53.6 and
+// 69.8 / 63.7 us), 4 limbs at 6 (83.3 / 84.0); n = 2^13, 4 limbs between 8 and 16
+// (61.7 / 65.5 and 97.6 / 92.4); n = 2^12, 12 limbs at 2 (71.6 / 74.1)).
+const shg::Ks32& ks32_for(const shg_context* ctx, const shg_key* key, int count, bool one_key) {
+  static const shg::Ks32 none;
+  const CtxDev c = ctx->dev();
+  if (!key->ks32.key || !one_key || !c.ks_fused || (c.log_n < c.ntt4_plain_min && c.log_n <= 14))
+    return none;
+  const double k = key->k, L = key->L;
+  const double saved = k * L - 0.45 * (3 * k + 6 * L) - 2 * L;
+  return saved * count * ctx->n >= 1.75e6 ? key->ks32 : none;
+}
+// Digit scratch of one ciphertext of a key switch through that form or without.
+// Workspaces hold the larger need of the two, so that a call of fewer
+// ciphertexts (which may take the other form) never needs more than one of more.
+size_t ks_scratch_bytes(const shg_context* ctx, const shg_key* key, const shg::Ks32& ks32) {
+  if (ks32.key) return shg::ks32_scratch_bytes(key->k, key->L) * ctx->n;
+  return (size_t)key->k * key->L * ctx->n * sizeof(uint64_t);
 }
 
 // Cts per pipeline chunk, bounded by the scratch budget.
@@ -548,6 +582,10 @@ void shg_context_destroy(shg_context* ctx) {
   cudaFree(ctx->d_qmod);
   cudaFree(ctx->ws);
   cudaFree(ctx->io);
+  for (shg_context::Set32& t : ctx->set32) {
+    cudaFree(t.d_tw);
+    cudaFree(t.d_crt);
+  }
   for (cudaStream_t s : ctx->io_streams)
     if (s) cudaStreamDestroy(s);
   for (cudaStream_t s : ctx->io_lanes)
@@ -829,9 +867,193 @@ int shg_ct_tensor(shg_context* ctx, uint64_t* out, const uint64_t* a,
   return launch_status("ct_tensor");
 }
 
+}  // extern "C"
+
 // ---------------------------------------------------------------------------
 // Keys and key switching
 // ---------------------------------------------------------------------------
+
+namespace {
+
+// The three largest primes below 2^bits that are 1 mod 2^16 (every ring degree
+// up to 2^15).
+void find_primes32(int bits, uint32_t p[3]) {
+  uint32_t c = (1u << bits) + 1;
+  for (int a = 0; a < 3;) {
+    c -= 1u << 16;
+    bool prime = true;
+    for (uint32_t d = 3; (uint64_t)d * d <= c && prime; d += 2) prime = c % d != 0;
+    if (prime) p[a++] = c;
+  }
+}
+
+// Tables of one set of auxiliary primes (under ctx->mu).  0 on success; a
+// failed allocation leaves the set unmade.
+int make_set32(shg_context* ctx, int lazy) {
+  shg_context::Set32& set = ctx->set32[lazy];
+  if (set.d_tw) return SHG_OK;
+  const int n = ctx->n, L = ctx->L, log_n = ctx->log_n;
+  shg::W32 w{};
+  uint32_t ps[3];
+  find_primes32(lazy ? 28 : 30, ps);
+  std::vector<uint2> tw((size_t)6 * n);
+  for (int a = 0; a < 3; ++a) {
+    const uint64_t p = ps[a];
+    shg::Pr32& d = w.pr[a];
+    d.p = ps[a];
+    d.p2 = 2 * ps[a];
+    d.p4 = 4 * ps[a];
+    d.p8 = 8 * ps[a];
+    uint32_t inv = (uint32_t)p;  // Newton: p^-1 mod 2^32
+    for (int i = 0; i < 5; ++i) inv *= 2 - (uint32_t)p * inv;
+    d.pinv = inv;
+    d.r = (uint32_t)(((uint64_t)1 << 32) % p);
+    d.bar = (uint32_t)(((uint64_t)1 << 32) / p);
+    w.finv[a] = (float)(1.0 / (double)p);
+    uint64_t cof = 1;  // P / p mod p
+    for (int b = 0; b < 3; ++b)
+      if (b != a) cof = cof * (ps[b] % p) % p;
+    d.scale = (uint32_t)((uint64_t)d.r * powmod((uint64_t)n * cof % p, p - 2, p) % p);
+    uint64_t psi = 0;
+    for (uint64_t t = 2; !psi; ++t) {
+      const uint64_t cand = powmod(t, (p - 1) / (2 * (uint64_t)n), p);
+      if (powmod(cand, (uint64_t)n, p) == p - 1) psi = cand;
+    }
+    const uint64_t psi_inv = powmod(psi, p - 2, p);
+    std::vector<uint32_t> pw(n + 1), pwi(n + 1);
+    pw[0] = pwi[0] = 1;
+    for (int e = 1; e <= n; ++e) {
+      pw[e] = (uint32_t)(pw[e - 1] * psi % p);
+      pwi[e] = (uint32_t)(pwi[e - 1] * psi_inv % p);
+    }
+    auto shoup32 = [&](uint32_t v) {
+      return make_uint2(v, (uint32_t)(((uint64_t)v << 32) / p));
+    };
+    for (int i = 0; i < n; ++i) {
+      const uint32_t b = bitrev((uint32_t)i, log_n);
+      tw[(size_t)a * n + i] = shoup32(pw[b]);
+      tw[(size_t)(3 + a) * n + i] = shoup32(pwi[b + 1]);
+    }
+  }
+  // Sums of products of a digit transform (below 2p lazily, else p) and a key
+  // value (below p), beside one folded sum (below 2^32 (p + 1)).
+  const uint64_t pm = ps[0];
+  w.chunk = (int)std::min<uint64_t>(
+      1 << 20, (~(uint64_t)0 - ((pm + 1) << 32)) / ((lazy ? 2 : 1) * pm * pm));
+  std::vector<shg::Crt32> crt(L);
+  for (int l = 0; l < L; ++l) {
+    const uint64_t q = ctx->hp[l].q;
+    for (int a = 0; a < 3; ++a) {
+      uint64_t v = 1;
+      for (int b = 0; b < 3; ++b)
+        if (b != a) v = mulmod(v, ps[b] % q, q);
+      crt[l].w[a] = v;
+      crt[l].wp[a] = shoup_of(v, q);
+    }
+    crt[l].neg_p = q - mulmod(crt[l].w[0], ps[0] % q, q);
+  }
+  cudaError_t e = cudaMalloc(&set.d_tw, sizeof(uint2) * tw.size());
+  if (e == cudaSuccess) e = cudaMalloc(&set.d_crt, sizeof(shg::Crt32) * L);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(set.d_tw, tw.data(), sizeof(uint2) * tw.size(), cudaMemcpyHostToDevice);
+  if (e == cudaSuccess)
+    e = cudaMemcpy(set.d_crt, crt.data(), sizeof(shg::Crt32) * L, cudaMemcpyHostToDevice);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(set.d_tw);
+    cudaFree(set.d_crt);
+    set.d_tw = nullptr;
+    set.d_crt = nullptr;
+    return SHG_RESOURCE_EXHAUSTED;
+  }
+  w.fwd = set.d_tw;
+  w.inv = set.d_tw + (size_t)3 * n;
+  set.w = w;
+  return SHG_OK;
+}
+
+// Gives the key (already on the device) its 32-bit form where launch_ks32 can
+// and should use it:
+//  - n = 2^12 .. 2^15 (its transforms) and at least kKs32MinLimbs limbs: with
+//    few limbs the reconstruction costs more than the digit transforms it saves;
+//  - plain digits of at most 26 bits (below every auxiliary prime, no lift);
+//  - primes below 2^57: the reconstruction enters the lazy 64-bit transform
+//    below 33 q, which grows by at most 60 q;
+//  - |S| <= n sum_j max(d_j) q_max / 2 below 0.499 P, for the lazy primes below
+//    2^28 (n <= 2^14: at most 7 levels per phase) or else those below 2^30;
+//  - at most 128 digits (one row of each in shared memory) and scratch no
+//    larger than the general path's digit transforms.
+// Without device memory for it the key works as it is.
+constexpr int kKs32MinLimbs = 4;
+void make_key32(shg_context* ctx, shg_key* key, const std::vector<DigitDesc>& dd) {
+  const int L = key->L, k = key->k, log_n = ctx->log_n;
+  const size_t n = ctx->n;
+  if (log_n < 12 || log_n > 15 || L < kKs32MinLimbs || key->digit_flags != 0) return;
+  if (*std::max_element(key->log_bs.begin(), key->log_bs.end()) > 26) return;
+  if (k > 128 || shg::ks32_scratch_bytes(k, L) > 8 * (size_t)k * L) return;
+  uint64_t qmax = 0;
+  for (int l = 0; l < L; ++l) qmax = std::max(qmax, ctx->hp[l].q);
+  if (qmax >> 57) return;
+  uint64_t digit_sum = 0;
+  for (const DigitDesc& d : dd)
+    digit_sum += std::min<uint64_t>(d.mask, ctx->hp[d.src_limb].q >> d.shift);
+  const u128 twice_s = (u128)digit_sum * n * qmax;  // 2 |S|
+  std::lock_guard<std::mutex> lock(ctx->mu);
+  int lazy = -1;
+  for (int z : {1, 0}) {
+    if (z && log_n > 14) continue;
+    uint32_t p[3];
+    find_primes32(z ? 28 : 30, p);
+    const u128 P = (u128)p[0] * p[1] * p[2];
+    if (twice_s < P / 1000 * 998) {
+      lazy = z;
+      break;
+    }
+  }
+  if (lazy < 0 || make_set32(ctx, lazy) != SHG_OK) return;
+  const size_t elems = (size_t)k * L * n;
+  uint64_t* rows = nullptr;
+  uint32_t *tmp = nullptr, *key32 = nullptr;
+  cudaError_t e = cudaMalloc(&rows, elems * sizeof(uint64_t));
+  if (e == cudaSuccess) e = cudaMalloc(&tmp, 3 * elems * sizeof(uint32_t));
+  // the row kernel fetches a few digits ahead of the last row's end
+  const size_t key_words = 6 * elems + (size_t)shg::kKs32PadDigits * L * 256;
+  if (e == cudaSuccess) e = cudaMalloc(&key32, key_words * sizeof(uint32_t));
+  if (e == cudaSuccess) {
+    const shg_context::Set32& set = ctx->set32[lazy];
+    const CtxDev dv = ctx->dev();
+    for (int c = 0; c < 2; ++c) {
+      // the stored rows carry 2^64 mod q: the export scaling takes it off
+      shg::launch_ntt_inv(dv, c ? key->ka : key->kb, rows, k * L, L, 1, 0);
+      shg::launch_ks32_key(dv, set.w, rows, tmp, k, L, c, key32, 0);
+    }
+    e = cudaDeviceSynchronize();
+  }
+  cudaFree(rows);
+  cudaFree(tmp);
+  if (e != cudaSuccess) {
+    cudaGetLastError();
+    cudaFree(key32);
+    return;
+  }
+  const shg_context::Set32& set = ctx->set32[lazy];
+  key->d_key32 = key32;
+  key->bytes += key_words * sizeof(uint32_t);
+  key->ks32.key = key32;
+  key->ks32.crt = set.d_crt;
+  key->ks32.lazy = lazy;
+  key->ks32.w = set.w;
+  int j = 0;
+  for (int l = 0; l < L; ++l) {
+    key->ks32.first.j[l] = (short)j;
+    while (j < k && dd[j].src_limb == l) ++j;
+  }
+  key->ks32.first.j[L] = (short)j;
+}
+
+}  // namespace
+
+extern "C" {
 
 int shg_key_create(shg_context* ctx, int num_limbs, const int* log_bs,
                    int power, const uint64_t* key_b, const uint64_t* key_a,
@@ -916,6 +1138,7 @@ int shg_key_create(shg_context* ctx, int num_limbs, const int* log_bs,
     shg_key_destroy(key);
     return cuda_fail(e, "key conversion");
   }
+  make_key32(ctx, key, dd);
   *out = key;
   return SHG_OK;
 }
@@ -924,6 +1147,7 @@ void shg_key_destroy(shg_key* key) {
   if (!key) return;
   cudaFree(key->kb);
   cudaFree(key->ka);
+  cudaFree(key->d_key32);
   cudaFree(key->d_digits);
   delete key;
 }
@@ -962,18 +1186,24 @@ int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
               const shg_key* const* keys = nullptr) {
   const int L = key->L, n = ctx->n, k = key->k;
   const size_t Ln = (size_t)L * n;
-  const size_t per_ct = (Ln + (size_t)k * Ln) * sizeof(uint64_t);
+  const shg::Ks32& ks32 = ks32_for(ctx, key, count, keys == nullptr);
+  const size_t d_per_ct = ks_scratch_bytes(ctx, key, ks32);
+  const size_t per_ct = Ln * sizeof(uint64_t) + d_per_ct;
+  const size_t per_ct_plain =
+      Ln * sizeof(uint64_t) + ks_scratch_bytes(ctx, key, shg::Ks32{});
   const int C = chunk_for(ctx, per_ct, count);
+  const size_t need =
+      std::max(per_ct * C, per_ct_plain * chunk_for(ctx, per_ct_plain, count));
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
   std::lock_guard<std::mutex> lock(ctx->mu);
-  int st = ctx->ensure_ws(per_ct * C + tab_bytes);
+  int st = ctx->ensure_ws(need + tab_bytes);
   if (st) return st;
   uint64_t* X = ctx->ws;
   uint64_t* D = X + (size_t)C * Ln;
   shg::KeyTable table;
   if (keys &&
       (st = upload_key_table(keys, count, 1, 0,
-                             reinterpret_cast<const uint64_t**>(D + (size_t)C * k * Ln),
+                             reinterpret_cast<const uint64_t**>(D + C * d_per_ct / 8),
                              &table, s)))
     return st;
   const CtxDev dv = ctx->dev();
@@ -987,7 +1217,7 @@ int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
     shg::launch_keyswitch(dv, D, X, key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
                           key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src,
                           (size_t)a.ncomp * Ln, CtMap::identity(), a.base1_zero,
-                          a.subst_power, cc, L, s, kt);
+                          a.subst_power, cc, L, s, kt, ks32);
   }
   return launch_status("keyswitch");
 }
@@ -1048,13 +1278,16 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
   // and the exported coefficients X of every degree-2 component.  Phase 2 in
   // chunks of the digit NTTs D and the key inner product.
   const size_t x_bytes = (size_t)count * Ln * sizeof(uint64_t);
-  const size_t d_per_ct = (size_t)k * Ln * sizeof(uint64_t);
+  const shg::Ks32& ks32 = ks32_for(ctx, key, count, keys == nullptr);
+  const size_t d_per_ct = ks_scratch_bytes(ctx, key, ks32);
   // 16 ciphertexts per chunk measured fastest at n = 2^14, L = 6 (the digit
   // kernel's grid is then ~13.8 K CTAs).
-  int C = ctx->chunk_cts > 0 ? ctx->chunk_cts
-                             : (int)std::max<size_t>(1, ((size_t)256 << 20) / d_per_ct);
-  C = std::min(C, 16);
-  C = std::max(1, std::min(C, count));
+  auto chunk_of = [&](size_t per_ct) {
+    int c = ctx->chunk_cts > 0 ? ctx->chunk_cts
+                               : (int)std::max<size_t>(1, ((size_t)256 << 20) / per_ct);
+    return std::max(1, std::min({c, 16, count}));
+  };
+  const int C = chunk_of(d_per_ct);
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
   std::lock_guard<std::mutex> lock(ctx->mu);
   // Chunks rotate over the caller's stream and up to three more (ks_lanes in
@@ -1071,14 +1304,20 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
     }
   }
   const int nchunks = (count + C - 1) / C;
-  const int lanes = ctx->ks_fork ? std::max(1, std::min(ctx->ks_lanes, nchunks)) : 1;
-  if ((st = ctx->ensure_ws(x_bytes + lanes * d_per_ct * C + tab_bytes))) return st;
+  auto lanes_of = [&](int c) {
+    return ctx->ks_fork ? std::max(1, std::min(ctx->ks_lanes, (count + c - 1) / c)) : 1;
+  };
+  const int lanes = lanes_of(C);
+  const size_t d_plain = ks_scratch_bytes(ctx, key, shg::Ks32{});
+  const size_t need =
+      std::max(lanes * d_per_ct * C, lanes_of(chunk_of(d_plain)) * d_plain * chunk_of(d_plain));
+  if ((st = ctx->ensure_ws(x_bytes + need + tab_bytes))) return st;
   uint64_t* X = ctx->ws;
   uint64_t* D0 = X + (size_t)count * Ln;
   shg::KeyTable kt;
   if (keys &&
       (st = upload_key_table(keys, count, 1, 0,
-                             reinterpret_cast<const uint64_t**>(D0 + (size_t)lanes * C * k * Ln),
+                             reinterpret_cast<const uint64_t**>(D0 + lanes * C * d_per_ct / 8),
                              &kt, s)))
     return st;
   const CtxDev dv = ctx->dev();
@@ -1095,10 +1334,10 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
     uint64_t* o = out + (size_t)c0 * 2 * Ln;
     shg::KeyTable kc;
     if (keys) kc = shg::KeyTable{kt.kb + c0, kt.ka + c0, 0, count - c0};
-    shg::launch_keyswitch(dv, D0 + (size_t)lane * C * k * Ln, X + (size_t)c0 * Ln,
+    shg::launch_keyswitch(dv, D0 + lane * C * d_per_ct / 8, X + (size_t)c0 * Ln,
                           key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
                           key->kb, key->ka, o, o, 2 * Ln, CtMap::identity(), 0, 0, cc, L, ls,
-                          kc);
+                          kc, ks32);
   }
   for (int i = 0; i + 1 < lanes; ++i) {
     SHG_CUDA(cudaEventRecord(ctx->ks_join[i], ctx->ks_side[i]));
@@ -1173,10 +1412,15 @@ int mul_relin_host_impl(shg_context* ctx, const shg_key* key, void* out_v, const
   const int S = ctx->host_slots;
   const size_t packed = wire ? 3 * (size_t)P * host_ct_pad : 0;
   const size_t slot = 3 * (size_t)P * ct_bytes + (size_t)P * Ln * sizeof(uint64_t) + packed;
-  const size_t d_per_ct = (size_t)k * Ln * sizeof(uint64_t);
-  int C = ctx->chunk_cts > 0 ? ctx->chunk_cts
-                             : (int)std::max<size_t>(1, ((size_t)256 << 20) / d_per_ct);
-  C = std::max(1, std::min({C, 16, P}));
+  const shg::Ks32& ks32 = ks32_for(ctx, key, count, true);
+  const size_t d_per_ct = ks_scratch_bytes(ctx, key, ks32);
+  auto chunk_of = [&](size_t per_ct) {
+    int c = ctx->chunk_cts > 0 ? ctx->chunk_cts
+                               : (int)std::max<size_t>(1, ((size_t)256 << 20) / per_ct);
+    return std::max(1, std::min({c, 16, P}));
+  };
+  const int C = chunk_of(d_per_ct);
+  const size_t d_plain = ks_scratch_bytes(ctx, key, shg::Ks32{});
   const int lanes = std::max(1, std::min(ctx->ks_lanes, (int)shg_context::kMaxKsLanes));
   std::lock_guard<std::mutex> io_lock(ctx->io_mu);
   std::lock_guard<std::mutex> lock(ctx->mu);
@@ -1192,7 +1436,8 @@ int mul_relin_host_impl(shg_context* ctx, const shg_key* key, void* out_v, const
     }
     ctx->io_bytes = S * slot;
   }
-  if ((st = ctx->ensure_ws((size_t)lanes * C * d_per_ct))) return st;
+  if ((st = ctx->ensure_ws(lanes * std::max(C * d_per_ct, chunk_of(d_plain) * d_plain))))
+    return st;
   uint64_t* D0 = ctx->ws;
   for (cudaStream_t& s : ctx->io_streams)
     if (!s) SHG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -1291,10 +1536,10 @@ int mul_relin_host_impl(shg_context* ctx, const shg_key* key, void* out_v, const
       if (!used[lane]) SHG_CUDA(cudaStreamWaitEvent(ls, tensored[i], 0));
       used[lane] = true;
       uint64_t* o = dout + (size_t)j * 2 * Ln;
-      shg::launch_keyswitch(dv, D0 + (size_t)lane * C * k * Ln, dx + (size_t)j * Ln,
+      shg::launch_keyswitch(dv, D0 + lane * C * d_per_ct / 8, dx + (size_t)j * Ln,
                             key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
                             key->kb, key->ka, o, o, 2 * Ln, CtMap::identity(), 0, 0, nc, L, ls,
-                            shg::KeyTable{});
+                            shg::KeyTable{}, ks32);
     }
     for (int lane = 0; lane < lanes; ++lane) {
       if (!used[lane]) continue;
@@ -1983,7 +2228,8 @@ int shg_debug_status(unsigned* first_failure) {
   if (!first_failure) return fail(SHG_INVALID_ARGUMENT, "null argument");
   const unsigned a = shg::take_debug_word_kernels();
   const unsigned b = shg::take_debug_word_ntt4();
-  *first_failure = a ? a : b;
+  const unsigned d = shg::take_debug_word_ks32();
+  *first_failure = a ? a : (b ? b : d);
   return SHG_OK;
 }
 
@@ -2537,7 +2783,8 @@ extern "C" int shg_relin_apply_noalloc(shg_context* ctx, const shg_key* key,
     shg::launch_intt_export(dv, X, src, 3, 2, 0, CtMap::identity(), cc, L, s);
     shg::launch_keyswitch(dv, D, X, key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
                           key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src, 3 * Ln,
-                          CtMap::identity(), 0, 0, cc, L, s);
+                          CtMap::identity(), 0, 0, cc, L, s, shg::KeyTable{},
+                          ks32_for(ctx, key, count, true));
   }
   return launch_status("relin_apply_noalloc");
 }

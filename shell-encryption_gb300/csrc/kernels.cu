@@ -1060,9 +1060,14 @@ void launch_keyswitch(const CtxDev& c, uint64_t* D, const uint64_t* X,
                       const uint64_t* kb, const uint64_t* ka, uint64_t* out,
                       const uint64_t* base, size_t base_ct_elems, CtMap map,
                       int base1_zero, int subst_power, int count, int L,
-                      cudaStream_t s, const KeyTable& kt) {
+                      cudaStream_t s, const KeyTable& kt, const Ks32& ks32) {
   if (count <= 0) return;
   const int need_lift = digit_flags & 1;
+  if (ks32.key) {
+    launch_ks32(c, ks32, D, X, digits, k, out, base, base_ct_elems, map, base1_zero, subst_power,
+                count, L, s);
+    return;
+  }
   if (use_ntt4(c) && c.ks_fused && ks4_rows_per_cta(k) > 0) {
     {
       LaunchScope scope_("digit_cols", s);

@@ -110,6 +110,7 @@ __device__ __forceinline__ I dbg_index(I idx, long long bound, unsigned tag) {
 // after reading (0: no check failed).
 unsigned take_debug_word_kernels();
 unsigned take_debug_word_ntt4();
+unsigned take_debug_word_ks32();
 
 // Number of kernels this library has launched (host-side counter).
 extern std::atomic<uint64_t> g_launch_count;
@@ -216,9 +217,65 @@ void launch_ks_inner(const CtxDev& c, uint64_t* out, const uint64_t* D,
                      int base1_zero, int subst_power, int count, int L,
                      cudaStream_t s, const KeyTable& kt = KeyTable{});
 
+// Key switch in three auxiliary primes below 2^30 (ks32.cu).  One set of
+// primes and tables per context and kind (lazy: below 2^28), passed to the
+// kernels by value.
+struct Pr32 {
+  uint32_t p, p2, p4, p8;  // p and its multiples 2p, 4p, 8p (8p wraps above 2^29: unused there)
+  uint32_t bar;            // floor(2^32 / p)
+  uint32_t pinv;           // p^-1 mod 2^32
+  uint32_t r;              // 2^32 mod p
+  uint32_t scale;          // 2^32 n^-1 (P/p)^-1 mod p: folded into imported keys
+};
+struct W32 {
+  Pr32 pr[3];
+  float finv[3];      // 1 / p
+  int chunk;          // inner-product terms per 64-bit accumulation
+  const uint2* fwd;   // [3][n] (psi^brv(i), Shoup constant)
+  const uint2* inv;   // [3][n] inverse twiddles in the reference's order
+};
+// Reconstruction modulo q_l: P/p_a mod q_l with Shoup constants, -P mod q_l.
+struct Crt32 {
+  uint64_t w[3], wp[3], neg_p, pad;
+};
+// Digits of limb l are j[l] .. j[l + 1] - 1 (DigitDesc order).
+struct Ks32Digits {
+  short j[kMaxLimbs + 1];
+};
+// Digits' worth of padding after a key (k32_rows fetches ahead).
+constexpr int kKs32PadDigits = 9;
+// A key in this form; key == nullptr: the key has none.
+struct Ks32 {
+  const uint32_t* key = nullptr;  // [3][n/128][k][L][2][128], padded
+  const Crt32* crt = nullptr;
+  int lazy = 0;
+  W32 w{};
+  Ks32Digits first{};
+};
+// Scratch bytes per ciphertext and coefficient: the digit transforms (their
+// space then holds the 64-bit sums), and all of it with the 32-bit sums.
+inline size_t ks32_digit_bytes(int k, int L) {
+  return 12 * (size_t)k > 16 * (size_t)L ? 12 * (size_t)k : 16 * (size_t)L;
+}
+inline size_t ks32_scratch_bytes(int k, int L) { return ks32_digit_bytes(k, L) + 24 * (size_t)L; }
+void launch_ks32(const CtxDev& c, const Ks32& ks, uint64_t* scratch, const uint64_t* X,
+                 const DigitDesc* digits, int k, uint64_t* out, const uint64_t* base,
+                 size_t base_ct_elems, CtMap map, int base1_zero, int subst_power, int count,
+                 int L, cudaStream_t s);
+// Imports component `comp` of a key: rows [k][L][n] in coefficient form, tmp
+// [k][L][3][n] scratch.
+void launch_ks32_key(const CtxDev& c, const W32& w, const uint64_t* rows, uint32_t* tmp, int k,
+                     int L, int comp, uint32_t* key, cudaStream_t s);
+// Row phase of the forward transforms buf [count][2][L][n] (column phase done)
+// plus the key switch's base: out [count][2][L][n].
+void launch4_rows_add(const CtxDev& c, const uint64_t* buf, uint64_t* out, const uint64_t* base,
+                      size_t base_ct_elems, CtMap map, int base1_zero, int subst_power,
+                      int count, int L, cudaStream_t s);
+
 // Gadget key switch core: digit decomposition + NTT of every digit + key
 // inner product + base add (launch_digit_ntt then launch_ks_inner).
-// D: [count][k][L][n] scratch.  digit_flags (digit_flags() below): bit 0 the
+// D: [count][k][L][n] scratch.  With a non-empty ks32 (one key for the batch)
+// launch_ks32 runs instead.  digit_flags (digit_flags() below): bit 0 the
 // digits need the balanced lift, bit 1 some digit is wider than 32 bits.
 inline int digit_flags(int need_lift, int max_log_b) {
   return (need_lift ? 1 : 0) | (max_log_b > 32 ? 2 : 0);
@@ -229,7 +286,8 @@ void launch_keyswitch(const CtxDev& c, uint64_t* D, const uint64_t* X,
                       const uint64_t* kb, const uint64_t* ka, uint64_t* out,
                       const uint64_t* base, size_t base_ct_elems, CtMap map,
                       int base1_zero, int subst_power, int count, int L,
-                      cudaStream_t s, const KeyTable& kt = KeyTable{});
+                      cudaStream_t s, const KeyTable& kt = KeyTable{},
+                      const Ks32& ks32 = Ks32{});
 
 // ModReduceLsb (NTT form): Y [count][n] scratch; out [count][L-1][n].
 // sc.v[4i..4i+3] = (c1, Shoup(c1), c2, Shoup(c2)) for output limb i with

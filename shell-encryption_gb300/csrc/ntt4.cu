@@ -243,6 +243,54 @@ struct FwdDstBgvEnc {
   }
 };
 
+// Key-switch sums plus their base (component (g / L) mod 2 of ciphertext
+// g / 2L): component 0 optionally read through X -> X^power, component 1
+// dropped when base1_zero.  base may be out (the same thread reads and writes
+// a position).
+template <int LOG_N>
+struct FwdDstKsBase {
+  static constexpr bool kTakesLazy = false;  // added to a canonical residue
+  uint64_t* out;
+  const uint64_t* base;
+  size_t base_ct_elems;
+  CtMap map;
+  int base1_zero, power, L;
+  struct H {
+    uint64_t* o;
+    const uint64_t* b;  // nullptr: no base
+    int power;
+    uint64_t q;
+    __device__ __forceinline__ uint64_t at(int i) const {
+      const unsigned j = __brev((unsigned)i) >> (32 - LOG_N);
+      const unsigned t = ((unsigned)((power - 1) >> 1) + j * (unsigned)power) &
+                         ((1u << LOG_N) - 1);
+      return b[dbg_index(__brev(t) >> (32 - LOG_N), 1LL << LOG_N, kDbgSubst)];
+    }
+    __device__ __forceinline__ void pair(int i, uint64_t x0, uint64_t x1) const {
+      ulonglong2 v = make_ulonglong2(0, 0);
+      if (power > 0)
+        v = make_ulonglong2(at(i), at(i + 1));
+      else if (b)
+        v = *reinterpret_cast<const ulonglong2*>(b + i);
+      *reinterpret_cast<ulonglong2*>(o + i) =
+          make_ulonglong2(add_mod(v.x, x0, q), add_mod(v.y, x1, q));
+    }
+  };
+  __device__ H bind(int g, int l, const CtxDev& c) const {
+    const int comp = (g / L) & 1;
+    const size_t p = (size_t)(g / (2 * L));
+    H h;
+    h.o = out + ((size_t)g << LOG_N);
+    h.b = comp && base1_zero
+              ? nullptr
+              : base + map(p) * base_ct_elems + (((size_t)comp * L + l) << LOG_N);
+    h.power = comp ? 0 : power;
+    h.q = c.primes[l].q;
+    return h;
+  }
+  __device__ void prefetch(int, int, int) const {}
+};
+
 // ---------------------------------------------------------------------------
 // Inverse phase-1 sources: the values at i, i + 1 of transform g (rows).
 // ---------------------------------------------------------------------------
@@ -1300,6 +1348,27 @@ void launch4_ks_rows(const CtxDev& c, const uint64_t* D, int k, int chunk,
     kern<<<count * L * ((1 << S::A) / R), threads, smem, s>>>(                  \
         D, k, R, chunk, kb, ka, out, base, base_ct_elems, map, base1_zero,      \
         subst_power, L, kt, c);                                                 \
+  }
+  SHG_DISPATCH4(c.log_n, F)
+#undef F
+}
+
+void launch4_rows_add(const CtxDev& c, const uint64_t* buf, uint64_t* out, const uint64_t* base,
+                      size_t base_ct_elems, CtMap map, int base1_zero, int subst_power,
+                      int count, int L, cudaStream_t s) {
+  // Three transforms of one prime per warp, one where the batch has only a
+  // ciphertext's two.
+#define F(LN)                                                                        \
+  {                                                                                  \
+    using Dst = FwdDstKsBase<LN>;                                                    \
+    const Dst dst{out, base, base_ct_elems, map, base1_zero, subst_power, L};        \
+    constexpr int W = kRowsWarpW;                                                    \
+    const int dpi = count == 1 ? 1 : kRowsWarpDpi;                                   \
+    const int groups = (2 * count + dpi - 1) / dpi;                                  \
+    auto kern = dpi == 1 ? k4_fwd_rows_warp<LN, true, Dst, W, 1>                     \
+                         : k4_fwd_rows_warp<LN, true, Dst, W, kRowsWarpDpi>;         \
+    kern<<<L * groups * (1 << (LN - 7)) / W, 32 * W, W * dpi * 128 * 8, s>>>(        \
+        buf, dst, PrimeMap{0, 1, L}, 2 * count * L, c);                              \
   }
   SHG_DISPATCH4(c.log_n, F)
 #undef F
