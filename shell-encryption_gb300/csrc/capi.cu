@@ -1824,6 +1824,10 @@ int run_expand(shg_context* ctx, const shg_key* const* keys, int levels, uint64_
       if (tables)
         kt = shg::KeyTable{tables[j].kb + q0, tables[j].ka + q0, j,
                            tables[j].entries ? tables[j].entries - q0 : 0};
+      if (shg::launch_ks_expand(dv, blk, D, X, key->d_digits, key->k, key->digit_flags, key->chunk,
+                                key->chunk_lazy, key->kb, key->ka, mono + (size_t)j * n, map, j,
+                                power, mc, s, kt))
+        continue;
       shg::launch_keyswitch(dv, D, X, key->d_digits, key->k, key->digit_flags,
                             key->chunk, key->chunk_lazy, key->kb, key->ka, KS, blk, 2 * (size_t)n,
                             map, 1, power, mc, 1, s, kt);

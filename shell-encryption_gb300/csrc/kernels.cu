@@ -626,6 +626,97 @@ __global__ void k_expand_combine(uint64_t* base, const uint64_t* ks,
   }
 }
 
+// Key inner product (k_ks_inner on one limb) and the level update of an
+// oblivious expansion (k_expand_combine) in one pass, in place.  Level j
+// substitutes by power n / 2^j + 1, which moves NTT index t to
+// t + n / 2^(j + 1) (1 + 2t): only its top j + 1 bits change, so in bit-reversed
+// order it permutes each aligned block of 2^(j + 1) positions.  A CTA owns
+// kExpandTile >= 2^(j + 1) positions of one member and reads every base value
+// before it writes one.  Two pairs of positions per thread keep six 16-byte loads in flight.
+// 512 members at n = 2^12, k = 8: 64 us against 56 + 22 as two kernels (the
+// key-switched member went through memory between them).
+constexpr int kExpandTile = 1024;
+__global__ void __launch_bounds__(256, 3)
+    k_ks_expand(uint64_t* base, const uint64_t* D, const uint64_t* kb, const uint64_t* ka, int k,
+                int chunk, const uint64_t* mono, CtMap map, int half, int power, int log_n,
+                KeyTable kt, CtxDev c) {
+  using V = ulonglong2;
+  constexpr int PT = kExpandTile / 512;  // pairs per thread
+  const size_t n = (size_t)1 << log_n, p = blockIdx.y;
+  if (kt.kb) {
+    const size_t e = dbg_index(p >> kt.shift, kt.entries ? kt.entries : (1LL << 62), kDbgKeyTable);
+    kb = kt.kb[e];
+    ka = kt.ka[e];
+  }
+  const uint64_t q = c.primes[0].q, qinv = c.primes[0].inv_modulus;
+  const int pos0 = blockIdx.x * kExpandTile + 2 * threadIdx.x;
+  const V* dp = reinterpret_cast<const V*>(D + p * k * n + pos0);
+  const V* bp = reinterpret_cast<const V*>(kb + pos0);
+  const V* ap = reinterpret_cast<const V*>(ka + pos0);
+  uint64_t s0[2 * PT], s1[2 * PT];
+#pragma unroll
+  for (int i = 0; i < 2 * PT; ++i) s0[i] = s1[i] = 0;
+  for (int j0 = 0; j0 < k; j0 += chunk) {
+    const int j1 = min(k, j0 + chunk);
+    uint64_t lo0[2 * PT], hi0[2 * PT], lo1[2 * PT], hi1[2 * PT];
+#pragma unroll
+    for (int i = 0; i < 2 * PT; ++i) lo0[i] = hi0[i] = lo1[i] = hi1[i] = 0;
+#pragma unroll 2
+    for (int j = j0; j < j1; ++j) {
+      V d[PT], vb[PT], va[PT];
+#pragma unroll
+      for (int i = 0; i < PT; ++i) {
+        d[i] = dp[256 * i];
+        vb[i] = __ldg(bp + 256 * i);
+        va[i] = __ldg(ap + 256 * i);
+      }
+#pragma unroll
+      for (int i = 0; i < PT; ++i) {
+        mac128(lo0[2 * i], hi0[2 * i], d[i].x, vb[i].x);
+        mac128(lo0[2 * i + 1], hi0[2 * i + 1], d[i].y, vb[i].y);
+        mac128(lo1[2 * i], hi1[2 * i], d[i].x, va[i].x);
+        mac128(lo1[2 * i + 1], hi1[2 * i + 1], d[i].y, va[i].y);
+      }
+      dp += n / 2;
+      bp += n / 2;
+      ap += n / 2;
+    }
+#pragma unroll
+    for (int i = 0; i < 2 * PT; ++i) {
+      s0[i] = add_mod(s0[i], redc128(lo0[i], hi0[i], q, qinv), q);
+      s1[i] = add_mod(s1[i], redc128(lo1[i], hi1[i], q, qinv), q);
+    }
+  }
+  uint64_t* cp = base + map(p) * 2 * n;
+  uint64_t* hp = cp + (size_t)half * 2 * n;
+  auto pair = [](uint64_t* x) -> V& { return *reinterpret_cast<V*>(x); };
+  V c0[PT], c1[PT];
+#pragma unroll
+  for (int i = 0; i < PT; ++i) {
+    const int pos = pos0 + 512 * i;
+    c0[i] = pair(cp + pos);
+    c1[i] = pair(cp + n + pos);
+#pragma unroll
+    for (int t = 0; t < 2; ++t)
+      s0[2 * i + t] = add_mod(cp[dbg_index(subst_src_rt(pos + t, power, log_n), 1LL << log_n,
+                                           kDbgSubst)],
+                              s0[2 * i + t], q);
+  }
+  __syncthreads();  // every base value of this tile is read
+#pragma unroll
+  for (int i = 0; i < PT; ++i) {
+    const int pos = pos0 + 512 * i;
+    const V m = __ldg(reinterpret_cast<const V*>(mono + pos));
+    const uint64_t *u0 = s0 + 2 * i, *u1 = s1 + 2 * i;
+    pair(hp + pos) = make_ulonglong2(mont_mul(sub_mod(c0[i].x, u0[0], q), m.x, q, qinv),
+                                     mont_mul(sub_mod(c0[i].y, u0[1], q), m.y, q, qinv));
+    pair(hp + n + pos) = make_ulonglong2(mont_mul(sub_mod(c1[i].x, u1[0], q), m.x, q, qinv),
+                                         mont_mul(sub_mod(c1[i].y, u1[1], q), m.y, q, qinv));
+    pair(cp + pos) = make_ulonglong2(add_mod(c0[i].x, u0[0], q), add_mod(c0[i].y, u0[1], q));
+    pair(cp + n + pos) = make_ulonglong2(add_mod(c1[i].x, u1[0], q), add_mod(c1[i].y, u1[1], q));
+  }
+}
+
 // Monomials -x^{n - 2^j}, j < levels, in coefficient form
 // (oblivious_expand.h:197-200): row j is zero but for coefficient n - 2^j,
 // which is `minus_one` (the Montgomery form of -1).
@@ -873,29 +964,50 @@ __global__ void k_scatter(uint64_t* const* dsts, const uint64_t* src, size_t ele
   }
 }
 
-// FusedAbsorbAddInPlace chain (symmetric_encryption.h:250-275).
-__global__ void k_absorb_sum(uint64_t* out, const uint64_t* cts,
-                             const uint64_t* db, int num_items,
-                             size_t item_stride, int chunk,
-                             size_t total /* count*2*n */, int log_n,
-                             CtxDev c) {
+// FusedAbsorbAddInPlace chain (symmetric_encryption.h:250-275): 64 positions
+// per CTA, the items dealt to eight warps whose canonical sums are added at the
+// end.  HBM-bound on the ciphertexts: 16 queries of 1024 items at n = 2^12 take
+// 202 us (1.07 GB; 497 us with one thread per position and all items).
+constexpr int kAbsorbSlices = 8;
+__global__ void __launch_bounds__(32 * kAbsorbSlices)
+    k_absorb_sum(uint64_t* out, const uint64_t* cts, const uint64_t* db, int num_items,
+                 size_t item_stride, int chunk, size_t total /* count*2*n */, int log_n,
+                 CtxDev c) {
+  __shared__ ulonglong2 part[kAbsorbSlices][32];
   const size_t n = (size_t)1 << log_n;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
+  const int lane = threadIdx.x & 31, slice = threadIdx.x >> 5;
+  const size_t e = ((size_t)blockIdx.x * 32 + lane) * 2;
   const uint64_t q = c.primes[0].q, qinv = c.primes[0].inv_modulus;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += stride) {
-    const size_t qi = e / (2 * n), r = e % (2 * n);
-    const size_t pos = r & (n - 1);
+  uint64_t s0 = 0, s1 = 0;
+  if (e < total) {
+    const size_t qi = e >> (log_n + 1), r = e & (2 * n - 1), pos = r & (n - 1);
     const uint64_t* cp = cts + qi * item_stride * 2 * n + r;
-    uint64_t s = 0;
-    for (int i0 = 0; i0 < num_items; i0 += chunk) {
-      const int i1 = min(num_items, i0 + chunk);
-      uint64_t lo = 0, hi = 0;
-      for (int i = i0; i < i1; ++i)
-        mac128(lo, hi, cp[(size_t)i * 2 * n], __ldg(db + (size_t)i * n + pos));
-      s = add_mod(s, redc128(lo, hi, q, qinv), q);
+    const uint64_t* dp = db + pos;
+    const int step = kAbsorbSlices * chunk;
+    for (int i0 = slice; i0 < num_items; i0 += step) {
+      const int i1 = (int)min((long long)num_items, (long long)i0 + step);
+      uint64_t lo0 = 0, hi0 = 0, lo1 = 0, hi1 = 0;
+#pragma unroll 4
+      for (int i = i0; i < i1; i += kAbsorbSlices) {
+        const ulonglong2 v = *reinterpret_cast<const ulonglong2*>(cp + (size_t)i * 2 * n);
+        const ulonglong2 d = __ldg(reinterpret_cast<const ulonglong2*>(dp + (size_t)i * n));
+        mac128(lo0, hi0, v.x, d.x);
+        mac128(lo1, hi1, v.y, d.y);
+      }
+      s0 = add_mod(s0, redc128(lo0, hi0, q, qinv), q);
+      s1 = add_mod(s1, redc128(lo1, hi1, q, qinv), q);
     }
-    out[e] = s;
+  }
+  part[slice][lane] = make_ulonglong2(s0, s1);
+  __syncthreads();
+  if (slice == 0 && e < total) {
+#pragma unroll
+    for (int t = 1; t < kAbsorbSlices; ++t) {
+      const ulonglong2 v = part[t][lane];
+      s0 = add_mod(s0, v.x, q);
+      s1 = add_mod(s1, v.y, q);
+    }
+    *reinterpret_cast<ulonglong2*>(out + e) = make_ulonglong2(s0, s1);
   }
 }
 
@@ -1228,6 +1340,21 @@ static dim3 ser_grid(const CtxDev& c, int count, int L) {
   return dim3(x, std::max(1, std::min(count, std::min(65535, c.sms * 32 / x + 1))));
 }
 
+bool launch_ks_expand(const CtxDev& c, uint64_t* base, uint64_t* D, const uint64_t* X,
+                      const DigitDesc* digits, int k, int digit_flags, int chunk, int chunk_lazy,
+                      const uint64_t* kb, const uint64_t* ka, const uint64_t* mono, CtMap map,
+                      int level, int power, int count, cudaStream_t s, const KeyTable& kt) {
+  if (use_ntt4(c) || c.n < kExpandTile || (2 << level) > kExpandTile || count > 65535)
+    return false;
+  if (count <= 0) return true;
+  launch_digit_ntt(c, D, X, digits, k, digit_flags, count, 1, s);
+  LaunchScope scope_("ks_expand", s);
+  k_ks_expand<<<dim3(c.n / kExpandTile, count), 256, 0, s>>>(
+      base, D, kb, ka, k, c.small_q ? chunk_lazy : chunk, mono, map, 1 << level, power, c.log_n,
+      kt, c);
+  return true;
+}
+
 void launch_deserialize(const CtxDev& c, uint64_t* polys, const uint8_t* in,
                         const SerLayout& lay, int count, int L, cudaStream_t s) {
   const size_t total = (size_t)count * L * c.n;
@@ -1317,8 +1444,8 @@ void launch_absorb_sum(const CtxDev& c, uint64_t* out, const uint64_t* cts,
   const size_t total = (size_t)count * 2 * c.n;
   if (total == 0) return;
   LaunchScope scope_("absorb_sum", s);
-  k_absorb_sum<<<grid_for(total, 256), 256, 0, s>>>(
-      out, cts, db, num_items, item_stride, chunk, total, c.log_n, c);
+  k_absorb_sum<<<(unsigned)((total / 2 + 31) / 32), 32 * kAbsorbSlices, 0, s>>>(
+      out, cts, db, num_items, item_stride, std::min(chunk, 1 << 20), total, c.log_n, c);
 }
 
 // Integer ceiling of the transforms: the NTT's lazy Cooley-Tukey butterfly

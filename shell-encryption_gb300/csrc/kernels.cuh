@@ -320,6 +320,14 @@ void launch_expand_combine(const CtxDev& c, uint64_t* base, const uint64_t* ks,
                            const uint64_t* mono, CtMap map, int half,
                            int count, cudaStream_t s);
 
+// One expansion level in place (digit NTTs, key inner product, update) of
+// members p (ciphertext at map(p) of base, exported component X) for `level`'s
+// power; false if this shape takes launch_keyswitch + launch_expand_combine.
+bool launch_ks_expand(const CtxDev& c, uint64_t* base, uint64_t* D, const uint64_t* X,
+                      const DigitDesc* digits, int k, int digit_flags, int chunk, int chunk_lazy,
+                      const uint64_t* kb, const uint64_t* ka, const uint64_t* mono, CtMap map,
+                      int level, int power, int count, cudaStream_t s, const KeyTable& kt);
+
 // One RNS basis conversion between two prime sets of a context
 // (RnsPolynomial::SwitchRnsBasis, ScaleAndSwitchRnsBasis, ApproxSwitchRnsBasis,
 // rns/rns_polynomial.cc:419-724), kept in device memory.  Source limb i's
