@@ -79,7 +79,8 @@ int shg_context_set_ks_fused(shg_context* ctx, int on);
  * on.  Reads and clears the current device's records: *first_failure = 0 when
  * no check failed.  A release build always reports 0. */
 int shg_debug_status(unsigned* first_failure);
-/* Streams the chunks of a batched ct-mult+relin rotate over, 1 to 4 (2 =
+/* Streams the chunks of a batched ct-mult+relin, rotation or key switch and the
+ * queries of an oblivious expansion rotate over, 1 to 4 (2 =
  * default: the caller's stream and a second one, so one chunk fills the
  * other's tail; 1 = the caller's stream only, e.g. to time kernels one at a
  * time).  Each lane holds its own chunk of digit scratch. */

@@ -1179,6 +1179,50 @@ struct KsArgs {
 int upload_key_table(const shg_key* const* keys, int count, int stride, int offset,
                      const uint64_t** dst, shg::KeyTable* out, cudaStream_t s);
 
+// Streams that the independent parts of one batched call rotate over: lane 0 is
+// the caller's, the others the context's (made outside any stream capture, by
+// the first call that wants them; without them there is one lane).  Parts on
+// other lanes fill the tails of each other's launches.  Under ctx->mu.
+struct KsLanes {
+  shg_context* ctx;
+  cudaStream_t s;
+  int n = 1;
+  // At most `want` lanes (and the context's setting).
+  int open(int want) {
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    SHG_CUDA(cudaStreamIsCapturing(s, &cap));
+    if (!ctx->ks_fork && std::min(want, ctx->ks_lanes) > 1 &&
+        cap == cudaStreamCaptureStatusNone) {
+      SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_fork, cudaEventDisableTiming));
+      for (int i = 0; i < shg_context::kMaxKsLanes - 1; ++i) {
+        SHG_CUDA(cudaStreamCreateWithFlags(&ctx->ks_side[i], cudaStreamNonBlocking));
+        SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_join[i], cudaEventDisableTiming));
+      }
+    }
+    n = lanes_of(want);
+    return SHG_OK;
+  }
+  int lanes_of(int want) const {
+    return ctx->ks_fork ? std::max(1, std::min(ctx->ks_lanes, want)) : 1;
+  }
+  cudaStream_t stream(int lane) const { return lane ? ctx->ks_side[lane - 1] : s; }
+  // The side lanes start after what is on lane 0 now; lane 0 goes on after them.
+  int fork() const {
+    if (n == 1) return SHG_OK;
+    SHG_CUDA(cudaEventRecord(ctx->ks_fork, s));
+    for (int i = 0; i + 1 < n; ++i)
+      SHG_CUDA(cudaStreamWaitEvent(ctx->ks_side[i], ctx->ks_fork, 0));
+    return SHG_OK;
+  }
+  int join() const {
+    for (int i = 0; i + 1 < n; ++i) {
+      SHG_CUDA(cudaEventRecord(ctx->ks_join[i], ctx->ks_side[i]));
+      SHG_CUDA(cudaStreamWaitEvent(s, ctx->ks_join[i], 0));
+    }
+    return SHG_OK;
+  }
+};
+
 // Gadget key switch of component a.comp of `count` ciphertexts; with `keys`,
 // member i uses keys[i] (same gadget shape as `key`).
 int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
@@ -1192,33 +1236,43 @@ int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
   const size_t per_ct_plain =
       Ln * sizeof(uint64_t) + ks_scratch_bytes(ctx, key, shg::Ks32{});
   const int C = chunk_for(ctx, per_ct, count);
-  const size_t need =
-      std::max(per_ct * C, per_ct_plain * chunk_for(ctx, per_ct_plain, count));
+  const int C_plain = chunk_for(ctx, per_ct_plain, count);
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
   std::lock_guard<std::mutex> lock(ctx->mu);
-  int st = ctx->ensure_ws(need + tab_bytes);
+  // Each lane has its own X and D; two chunks side by side measured 17 % faster
+  // (250 rotations at n = 2^14, six limbs: 2971 -> 2268 us).
+  KsLanes lanes{ctx, s};
+  const int nchunks = (count + C - 1) / C;
+  int st = lanes.open(nchunks);
   if (st) return st;
-  uint64_t* X = ctx->ws;
-  uint64_t* D = X + (size_t)C * Ln;
+  const size_t lane_bytes = per_ct * C;
+  const size_t need =
+      std::max(lanes.n * lane_bytes, lanes.lanes_of((count + C_plain - 1) / C_plain) *
+                                         (per_ct_plain * C_plain));
+  if ((st = ctx->ensure_ws(need + tab_bytes))) return st;
   shg::KeyTable table;
-  if (keys &&
-      (st = upload_key_table(keys, count, 1, 0,
-                             reinterpret_cast<const uint64_t**>(D + C * d_per_ct / 8),
-                             &table, s)))
+  if (keys && (st = upload_key_table(keys, count, 1, 0,
+                                     reinterpret_cast<const uint64_t**>(
+                                         ctx->ws + lanes.n * lane_bytes / sizeof(uint64_t)),
+                                     &table, s)))
     return st;
   const CtxDev dv = ctx->dev();
-  for (int c0 = 0; c0 < count; c0 += C) {
-    const int cc = std::min(C, count - c0);
+  if ((st = lanes.fork())) return st;
+  for (int i = 0; i < nchunks; ++i) {
+    const int c0 = i * C, cc = std::min(C, count - c0), lane = i % lanes.n;
+    uint64_t* X = ctx->ws + lane * lane_bytes / sizeof(uint64_t);
+    uint64_t* D = X + (size_t)C * Ln;
     const uint64_t* src = a.ct + (size_t)c0 * a.ncomp * Ln;
     shg::launch_intt_export(dv, X, src, a.ncomp, a.comp, a.subst_power,
-                            CtMap::identity(), cc, L, s);
+                            CtMap::identity(), cc, L, lanes.stream(lane));
     shg::KeyTable kt;
     if (keys) kt = shg::KeyTable{table.kb + c0, table.ka + c0, 0, count - c0};
     shg::launch_keyswitch(dv, D, X, key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
                           key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src,
                           (size_t)a.ncomp * Ln, CtMap::identity(), a.base1_zero,
-                          a.subst_power, cc, L, s, kt, ks32);
+                          a.subst_power, cc, L, lanes.stream(lane), kt, ks32);
   }
+  if ((st = lanes.join())) return st;
   return launch_status("keyswitch");
 }
 
@@ -1290,27 +1344,15 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
   const int C = chunk_of(d_per_ct);
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
   std::lock_guard<std::mutex> lock(ctx->mu);
-  // Chunks rotate over the caller's stream and up to three more (ks_lanes in
-  // all), each lane with its own digit scratch, so one chunk's kernels fill
-  // another's tail.  The extra streams are created outside any stream
-  // capture (the first call).
-  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-  SHG_CUDA(cudaStreamIsCapturing(s, &cap));
-  if (!ctx->ks_fork && cap == cudaStreamCaptureStatusNone) {
-    SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_fork, cudaEventDisableTiming));
-    for (int i = 0; i < shg_context::kMaxKsLanes - 1; ++i) {
-      SHG_CUDA(cudaStreamCreateWithFlags(&ctx->ks_side[i], cudaStreamNonBlocking));
-      SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_join[i], cudaEventDisableTiming));
-    }
-  }
+  // Chunks rotate over the lanes, each with its own digit scratch.
+  KsLanes ks_lanes{ctx, s};
   const int nchunks = (count + C - 1) / C;
-  auto lanes_of = [&](int c) {
-    return ctx->ks_fork ? std::max(1, std::min(ctx->ks_lanes, (count + c - 1) / c)) : 1;
-  };
-  const int lanes = lanes_of(C);
+  if ((st = ks_lanes.open(nchunks))) return st;
+  const int lanes = ks_lanes.n;
   const size_t d_plain = ks_scratch_bytes(ctx, key, shg::Ks32{});
   const size_t need =
-      std::max(lanes * d_per_ct * C, lanes_of(chunk_of(d_plain)) * d_plain * chunk_of(d_plain));
+      std::max(lanes * d_per_ct * C, ks_lanes.lanes_of((count + chunk_of(d_plain) - 1) / chunk_of(d_plain)) * d_plain *
+                   chunk_of(d_plain));
   if ((st = ctx->ensure_ws(x_bytes + need + tab_bytes))) return st;
   uint64_t* X = ctx->ws;
   uint64_t* D0 = X + (size_t)count * Ln;
@@ -1322,15 +1364,11 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
     return st;
   const CtxDev dv = ctx->dev();
   shg::launch_tensor_intt(dv, out, X, a, b, count, L, s);
-  if (lanes > 1) {
-    SHG_CUDA(cudaEventRecord(ctx->ks_fork, s));
-    for (int i = 0; i + 1 < lanes; ++i)
-      SHG_CUDA(cudaStreamWaitEvent(ctx->ks_side[i], ctx->ks_fork, 0));
-  }
+  if ((st = ks_lanes.fork())) return st;
   for (int i = 0; i < nchunks; ++i) {
     const int c0 = i * C, cc = std::min(C, count - c0);
     const int lane = i % lanes;
-    cudaStream_t ls = lane ? ctx->ks_side[lane - 1] : s;
+    cudaStream_t ls = ks_lanes.stream(lane);
     uint64_t* o = out + (size_t)c0 * 2 * Ln;
     shg::KeyTable kc;
     if (keys) kc = shg::KeyTable{kt.kb + c0, kt.ka + c0, 0, count - c0};
@@ -1339,10 +1377,7 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
                           key->kb, key->ka, o, o, 2 * Ln, CtMap::identity(), 0, 0, cc, L, ls,
                           kc, ks32);
   }
-  for (int i = 0; i + 1 < lanes; ++i) {
-    SHG_CUDA(cudaEventRecord(ctx->ks_join[i], ctx->ks_side[i]));
-    SHG_CUDA(cudaStreamWaitEvent(s, ctx->ks_join[i], 0));
-  }
+  if ((st = ks_lanes.join())) return st;
   return launch_status("bgv_mul_relin");
 }
 
@@ -1768,18 +1803,20 @@ int check_expand(const shg_context* ctx, const shg_key* const* keys, int levels,
 // 2^(levels-1) members one query contributes at the last level.
 struct ExpandPlan {
   int C = 1;
+  int lanes = 1;  // each with room for C members
   size_t mono_bytes = 0, per_member = 0;
-  size_t bytes() const { return mono_bytes + per_member * C; }
+  size_t bytes() const { return mono_bytes + lanes * per_member * C; }
 };
 
 ExpandPlan plan_expand(const shg_context* ctx, const shg_key* const* keys, int levels,
-                       int count) {
+                       int count, int lanes) {
   ExpandPlan p;
+  p.lanes = lanes;
   const int n = ctx->n;
   const int kmax = levels ? keys[0]->k : 0;
   p.per_member = ((size_t)n + (size_t)kmax * n + 2 * (size_t)n) * sizeof(uint64_t);
   p.mono_bytes = (size_t)levels * n * sizeof(uint64_t);
-  const int members_max = std::max(1, count << std::max(levels - 1, 0));
+  const int members_max = std::max(1, (count + lanes - 1) / lanes << std::max(levels - 1, 0));
   p.C = std::max(1 << std::max(levels - 1, 0),
                  (int)std::min<size_t>((size_t)members_max, ((size_t)256 << 20) / p.per_member));
   return p;
@@ -1801,41 +1838,52 @@ int run_expand(shg_context* ctx, const shg_key* const* keys, int levels, uint64_
   const int kmax = keys[0]->k;
   const size_t per_query = ((size_t)2 * n) << levels;
   uint64_t* mono = ws;
-  uint64_t* X = mono + (size_t)levels * n;
-  uint64_t* D = X + (size_t)C * n;
-  uint64_t* KS = D + (size_t)C * kmax * n;
   // Monomials -x^{n - 2^j} in NTT form (oblivious_expand.h:197-200), built
   // on the stream so the whole expansion can be captured in a graph.
   shg::launch_monomials(ctx->dev(), mono, levels, ctx->hp[0].q - ctx->hp[0].r_mod_q, s);
   shg::launch_ntt_fwd(ctx->dev(), mono, mono, levels, 1, s);
   const CtxDev dv = ctx->dev();
-  for (int j = 0; j < levels; ++j) {
-    const shg_key* key = keys[j];
-    const int power = (n >> j) + 1;
-    const CtMap map{j, levels};
-    // Members of a level are processed in chunks of whole queries.
-    const int q_per_chunk = std::max(1, C >> j);
-    for (int q0 = 0; q0 < count; q0 += q_per_chunk) {
-      const int qc = std::min(q_per_chunk, count - q0);
-      const int mc = qc << j;
-      uint64_t* blk = out + (size_t)q0 * per_query;
-      shg::launch_intt_export(dv, X, blk, 2, 1, power, map, mc, 1, s);
-      shg::KeyTable kt;
-      if (tables)
-        kt = shg::KeyTable{tables[j].kb + q0, tables[j].ka + q0, j,
-                           tables[j].entries ? tables[j].entries - q0 : 0};
-      if (shg::launch_ks_expand(dv, blk, D, X, key->d_digits, key->k, key->digit_flags, key->chunk,
-                                key->chunk_lazy, key->kb, key->ka, mono + (size_t)j * n, map, j,
-                                power, mc, s, kt))
-        continue;
-      shg::launch_keyswitch(dv, D, X, key->d_digits, key->k, key->digit_flags,
-                            key->chunk, key->chunk_lazy, key->kb, key->ka, KS, blk, 2 * (size_t)n,
-                            map, 1, power, mc, 1, s, kt);
-      shg::launch_expand_combine(dv, blk, KS, mono + (size_t)j * n, map, 1 << j,
-                                 mc, s);
+  // Queries are independent: each lane takes its share of them through all
+  // levels with its own X, D and KS, so one lane's memory-bound level update
+  // runs beside another's digit transforms (24 queries of 10 levels at
+  // n = 2^12: 12.8 -> 11.3 ms).
+  KsLanes lanes{ctx, s, plan.lanes};
+  int st = lanes.fork();
+  if (st) return st;
+  const int share = (count + plan.lanes - 1) / plan.lanes;
+  for (int lane = 0; lane < plan.lanes; ++lane) {
+    const int first = lane * share, last = std::min(count, first + share);
+    cudaStream_t ls = lanes.stream(lane);
+    uint64_t* X = mono + (size_t)levels * n + lane * plan.per_member * C / sizeof(uint64_t);
+    uint64_t* D = X + (size_t)C * n;
+    uint64_t* KS = D + (size_t)C * kmax * n;
+    for (int j = 0; j < levels; ++j) {
+      const shg_key* key = keys[j];
+      const int power = (n >> j) + 1;
+      const CtMap map{j, levels};
+      // Members of a level are processed in chunks of whole queries.
+      const int q_per_chunk = std::max(1, C >> j);
+      for (int q0 = first; q0 < last; q0 += q_per_chunk) {
+        const int qc = std::min(q_per_chunk, last - q0);
+        const int mc = qc << j;
+        uint64_t* blk = out + (size_t)q0 * per_query;
+        shg::launch_intt_export(dv, X, blk, 2, 1, power, map, mc, 1, ls);
+        shg::KeyTable kt;
+        if (tables)
+          kt = shg::KeyTable{tables[j].kb + q0, tables[j].ka + q0, j,
+                             tables[j].entries ? tables[j].entries - q0 : 0};
+        if (shg::launch_ks_expand(dv, blk, D, X, key->d_digits, key->k, key->digit_flags,
+                                  key->chunk, key->chunk_lazy, key->kb, key->ka,
+                                  mono + (size_t)j * n, map, j, power, mc, ls, kt))
+          continue;
+        shg::launch_keyswitch(dv, D, X, key->d_digits, key->k, key->digit_flags, key->chunk,
+                              key->chunk_lazy, key->kb, key->ka, KS, blk, 2 * (size_t)n, map, 1,
+                              power, mc, 1, ls, kt);
+        shg::launch_expand_combine(dv, blk, KS, mono + (size_t)j * n, map, 1 << j, mc, ls);
+      }
     }
   }
-  return SHG_OK;
+  return lanes.join();
 }
 
 int absorb_chunk(const shg_context* ctx) {
@@ -1865,10 +1913,12 @@ int pir_impl(shg_context* ctx, const shg_key* const* keys, bool per_query_keys, 
   // a 1 GiB scratch region and are absorbed before the next group starts.
   const int group = (int)std::max<size_t>(
       1, std::min<size_t>((size_t)count, ((size_t)1 << 30) / (per_query_elems * 8)));
-  const ExpandPlan plan = plan_expand(ctx, keys, levels, group);
+  std::lock_guard<std::mutex> lock(ctx->mu);
+  KsLanes lanes{ctx, s};
+  if ((st = lanes.open(group))) return st;
+  const ExpandPlan plan = plan_expand(ctx, keys, levels, group, lanes.n);
   const size_t blocks_bytes = (size_t)group * per_query_elems * sizeof(uint64_t);
   const size_t tab_bytes = per_query_keys ? 2 * (size_t)levels * count * sizeof(void*) : 0;
-  std::lock_guard<std::mutex> lock(ctx->mu);
   if ((st = ctx->ensure_ws(plan.bytes() + blocks_bytes + tab_bytes))) return st;
   uint64_t* blocks = ctx->ws + plan.bytes() / sizeof(uint64_t);
   std::vector<shg::KeyTable> tables(per_query_keys ? levels : 0);
@@ -1920,8 +1970,10 @@ int shg_oblivious_expand(shg_context* ctx, const shg_key* const* keys,
                              2 * n * sizeof(uint64_t), cudaMemcpyDeviceToDevice, s));
   }
   if (levels == 0) return SHG_OK;
-  const ExpandPlan plan = plan_expand(ctx, keys, levels, count);
   std::lock_guard<std::mutex> lock(ctx->mu);
+  KsLanes lanes{ctx, s};
+  if ((st = lanes.open(count))) return st;
+  const ExpandPlan plan = plan_expand(ctx, keys, levels, count, lanes.n);
   if ((st = ctx->ensure_ws(plan.bytes()))) return st;
   if ((st = run_expand(ctx, keys, levels, out, count, plan, ctx->ws, s))) return st;
   return launch_status("oblivious_expand");
