@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <cmath>
 #include <cstdlib>
 #include <cstdio>
 #include <cstring>
@@ -2339,6 +2340,18 @@ static int check_variance(int variance) {
 
 static size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 
+// Scratch of the side-by-side sampler, 0 where the sequential one runs: it
+// pays while less than one of a ciphertext's uniform words is rejected on
+// average (half of a 45-bit prime's ciphertexts in 200 have one, all of a prime's
+// just above a power of two have n).
+static size_t reject_bytes(const shg_context* ctx, int L, int count) {
+  if (ctx->n < 64) return 0;
+  double expected = 0;
+  for (int l = 0; l < L; ++l)
+    expected += ctx->n * (1.0 - (double)ctx->hp[l].q / std::ldexp(1.0, ctx->hp[l].log_q));
+  return expected < 1 ? round256(count * shg::sample_reject_bytes()) : 0;
+}
+
 int shg_sample_uniform_error(shg_context* ctx, uint64_t* a, uint64_t* e,
                              const uint8_t* seeds, int num_limbs, int count, int variance,
                              shg_stream stream) {
@@ -2351,10 +2364,14 @@ int shg_sample_uniform_error(shg_context* ctx, uint64_t* a, uint64_t* e,
   const int L = num_limbs;
   const size_t Ln = (size_t)L * ctx->n;
   std::lock_guard<std::mutex> lock(ctx->mu);
-  if ((st = ctx->ensure_ws(round256((size_t)count * ctx->n * sizeof(int32_t))))) return st;
+  const size_t err_bytes = round256((size_t)count * ctx->n * sizeof(int32_t));
+  const size_t rej_bytes = reject_bytes(ctx, L, count);
+  if ((st = ctx->ensure_ws(err_bytes + rej_bytes))) return st;
   int32_t* err = reinterpret_cast<int32_t*>(ctx->ws);
   const shg::CtxDev dev = ctx->dev();
-  shg::launch_sample_uniform_error(dev, a, Ln, 0, err, seeds, L, variance, count, s);
+  shg::launch_sample_uniform_error(
+      dev, a, Ln, 0, err, seeds, L, variance, count,
+      rej_bytes ? reinterpret_cast<uint8_t*>(ctx->ws) + err_bytes : nullptr, s);
   shg::launch_error_lift(dev, e, err, count, L, s);
   shg::launch_ntt_fwd(dev, e, e, count * L, L, s);
   return launch_status("sample_uniform_error");
@@ -2384,13 +2401,15 @@ int shg_bgv_encrypt(shg_context* ctx, uint64_t* out, const uint64_t* key,
   const int C = (int)std::max<size_t>(1, std::min<size_t>((size_t)count, want));
   const size_t err_bytes = round256((size_t)count * n * sizeof(int32_t));
   std::lock_guard<std::mutex> lock(ctx->mu);
-  if ((st = ctx->ensure_ws(err_bytes + (size_t)C * per_ct))) return st;
+  const size_t rej_bytes = reject_bytes(ctx, L, count);
+  if ((st = ctx->ensure_ws(err_bytes + rej_bytes + (size_t)C * per_ct))) return st;
   int32_t* err = reinterpret_cast<int32_t*>(ctx->ws);
-  uint64_t* buf = reinterpret_cast<uint64_t*>(reinterpret_cast<uint8_t*>(ctx->ws) + err_bytes);
+  uint8_t* rej = reinterpret_cast<uint8_t*>(ctx->ws) + err_bytes;
+  uint64_t* buf = reinterpret_cast<uint64_t*>(rej + rej_bytes);
   const shg::CtxDev dev = ctx->dev();
   // c1 = -a straight from the sampler; the error waits in err.
   shg::launch_sample_uniform_error(dev, out + Ln, 2 * Ln, 1, err, seeds, L, variance, count,
-                                   s);
+                                   rej_bytes ? rej : nullptr, s);
   for (int c0 = 0; c0 < count; c0 += C) {
     const int cc = std::min(C, count - c0);
     uint64_t* o = out + (size_t)c0 * 2 * Ln;

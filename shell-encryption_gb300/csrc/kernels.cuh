@@ -416,10 +416,13 @@ int set_error(int code, const std::string& msg);
 // BGV encryption randomness from the ChaCha PRNG of seeds [count][32]
 // (RnsPolynomial::SampleUniform then SampleError): ciphertext p's uniform
 // polynomial (negated when `negate`) goes to a_dst + p * a_stride as [L][n],
-// its signed error coefficients to err [count][n].
+// its signed error coefficients to err [count][n].  rejects: scratch of
+// sample_reject_bytes() per ciphertext to sample all blocks side by side (for
+// primes that reject rarely; n >= 64), or nullptr for the sequential scan.
 void launch_sample_uniform_error(const CtxDev& c, uint64_t* a_dst, size_t a_stride,
                                  int negate, int32_t* err, const uint8_t* seeds, int L,
-                                 int variance, int count, cudaStream_t s);
+                                 int variance, int count, void* rejects, cudaStream_t s);
+size_t sample_reject_bytes();
 // Stream bytes one error coefficient of this variance takes.
 int sample_error_bytes(int variance);
 // out [count][L][n] <- err [count][n] lifted to every limb (Montgomery).

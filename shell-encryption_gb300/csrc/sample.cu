@@ -71,7 +71,7 @@ __device__ __forceinline__ void chacha_block(const uint32_t (&key)[8], uint32_t 
 __device__ __forceinline__ uint64_t word0(uint64_t g) {
   return (g >> 7) * kSaltWords + (g & 127) * 8;
 }
-__device__ __forceinline__ uint64_t block_of_word(uint64_t w) {
+__host__ __device__ __forceinline__ uint64_t block_of_word(uint64_t w) {
   return (w / kSaltWords) * 128 + (w % kSaltWords) / 8;
 }
 __device__ __forceinline__ uint64_t block_of_byte(uint64_t b) {
@@ -117,26 +117,101 @@ __device__ __forceinline__ int block_scan(int v, int* warp_sums, int* total) {
 // the in-order copy-out both run without shared-memory bank conflicts.
 __device__ __forceinline__ int stage_slot(int r) { return r ^ ((r >> 4) & 15); }
 
+__device__ __forceinline__ void load_seed(const uint8_t* seeds, int p, uint32_t (&key)[8]) {
+  const uint4* sp = reinterpret_cast<const uint4*>(seeds + (size_t)p * 32);
+  const uint4 k0 = sp[0], k1 = sp[1];
+  key[0] = k0.x; key[1] = k0.y; key[2] = k0.z; key[3] = k0.w;
+  key[4] = k1.x; key[5] = k1.y; key[6] = k1.z; key[7] = k1.w;
+}
+
+// Rejected words of one ciphertext's uniform part; a count above kMaxRejects
+// hands the ciphertext to the sequential kernel.
+constexpr unsigned kMaxRejects = 15;
+struct Rejects {
+  unsigned count;
+  unsigned word[kMaxRejects];
+};
+
+// Error coefficients per CTA pass: as many as THREADS * 64 bytes of keystream hold.
+template <int THREADS>
+__host__ __device__ __forceinline__ int error_per_pass(int k2) {
+  return THREADS * 64 / error_bytes(k2);
+}
+
+// Error coefficients j0 .. j0 + J - 1 of one ciphertext into err: coefficient j
+// takes stream bytes [e0 + j * B, e0 + (j + 1) * B), kept in `bytes` (shared, at
+// least THREADS * 64) between their generation and the counting.
+template <int THREADS>
+__device__ __forceinline__ void error_pass(uint8_t* bytes, const uint32_t (&key)[8], uint64_t e0,
+                                           int j0, int J, int k2, int32_t* err) {
+  const int tid = threadIdx.x, B = error_bytes(k2);
+  const uint64_t r0 = e0 + (uint64_t)j0 * B, r1 = r0 + (uint64_t)J * B;
+  const uint64_t gb0 = block_of_byte(r0), gb1 = block_of_byte(r1 - 1);
+  for (uint64_t g = gb0 + tid; g <= gb1; g += THREADS) {
+    uint32_t x[16];
+    chacha_block(key, (uint32_t)(g & 127), g >> 7, x);
+    const uint64_t b0 = (g >> 7) * kSaltBytes + (g & 127) * 64;
+    const int len = (g & 127) == 127 ? 32 : 64;
+    const uint64_t lo = max(b0, r0), hi = min(b0 + len, r1);
+    if (((lo | hi) & 3) == 0 && ((b0 - r0) & 3) == 0) {
+      // whole 32-bit words (block starts are 32-byte aligned)
+      uint32_t* words = reinterpret_cast<uint32_t*>(bytes);
+      for (uint64_t b = lo; b < hi; b += 4) words[(b - r0) >> 2] = x[(b - b0) >> 2];
+    } else {
+      for (uint64_t b = lo; b < hi; ++b) {
+        const uint32_t w = x[(b - b0) >> 2];
+        bytes[b - r0] = (uint8_t)(w >> (8 * ((b - b0) & 3)));
+      }
+    }
+  }
+  __syncthreads();
+  for (int j = tid; j < J; j += THREADS) {
+    const uint8_t* cb = bytes + (size_t)j * B;
+    int val = 0, kk = k2;
+    while (kk > 0) {
+      if (kk >= 64) {
+        uint64_t plus = 0, minus = 0;
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          plus |= (uint64_t)cb[i] << (8 * i);
+          minus |= (uint64_t)cb[8 + i] << (8 * i);
+        }
+        val += __popcll(plus) - __popcll(minus);
+        cb += 16;
+        kk -= 64;
+      } else if (kk >= 8) {
+        val += __popc(cb[0]) - __popc(cb[1]);
+        cb += 2;
+        kk -= 8;
+      } else {
+        const unsigned m = (1u << kk) - 1;
+        val += __popc(cb[0] & m) - __popc(cb[1] & m);
+        break;
+      }
+    }
+    err[j0 + j] = val;
+  }
+}
+
 // One CTA of THREADS threads per ciphertext p.  a (uniform, Montgomery
 // values; negated when `negate`, i.e. written as c1 = -a) goes to
 // a_dst + p * a_stride as [L][n]; the signed error coefficients to err [p][n].
+// rejects: nullptr, or the records of k_sample_guess / k_sample_fix, of which
+// this kernel does the ciphertexts that they gave up on.
 template <int THREADS>
 __global__ void __launch_bounds__(THREADS)
     k_sample_uniform_error(uint64_t* a_dst, size_t a_stride, int negate, int32_t* err,
-                           const uint8_t* seeds, int L, int variance, int log_n, CtxDev c) {
+                           const uint8_t* seeds, int L, int variance, int log_n,
+                           const Rejects* rejects, CtxDev c) {
   constexpr int kStageWords = THREADS * 8;
   __shared__ uint64_t stage[kStageWords];  // accepted words / error keystream bytes
   __shared__ int warp_sums[THREADS / 32];
   __shared__ unsigned long long s_stop;
   const int p = blockIdx.x, tid = threadIdx.x;
+  if (rejects && rejects[p].count <= kMaxRejects) return;
   const int n = 1 << log_n;
   uint32_t key[8];
-  {
-    const uint4* sp = reinterpret_cast<const uint4*>(seeds + (size_t)p * 32);
-    const uint4 k0 = sp[0], k1 = sp[1];
-    key[0] = k0.x; key[1] = k0.y; key[2] = k0.z; key[3] = k0.w;
-    key[4] = k1.x; key[5] = k1.y; key[6] = k1.z; key[7] = k1.w;
-  }
+  load_seed(seeds, p, key);
   uint64_t pos = 0;  // next candidate word of the stream
   for (int l = 0; l < L; ++l) {
     const PrimeDev& P = c.primes[l];
@@ -190,63 +265,157 @@ __global__ void __launch_bounds__(THREADS)
     }
   }
 
-  // Error coefficients: coefficient j takes stream bytes
-  // [e0 + j * B, e0 + (j + 1) * B), e0 = 8 * pos.
-  const int k2 = 2 * variance;
-  const int B = error_bytes(k2);
-  const int per_pass = (kStageWords * 8) / B;
-  uint8_t* bytes = reinterpret_cast<uint8_t*>(stage);
   const uint64_t e0 = pos * 8;
+  const int k2 = 2 * variance, per_pass = error_per_pass<THREADS>(k2);
   for (int j0 = 0; j0 < n; j0 += per_pass) {
-    const int J = min(per_pass, n - j0);
-    const uint64_t r0 = e0 + (uint64_t)j0 * B, r1 = r0 + (uint64_t)J * B;
-    const uint64_t gb0 = block_of_byte(r0), gb1 = block_of_byte(r1 - 1);
-    for (uint64_t g = gb0 + tid; g <= gb1; g += THREADS) {
-      uint32_t x[16];
-      chacha_block(key, (uint32_t)(g & 127), g >> 7, x);
-      const uint64_t b0 = (g >> 7) * kSaltBytes + (g & 127) * 64;
-      const int len = (g & 127) == 127 ? 32 : 64;
-      const uint64_t lo = max(b0, r0), hi = min(b0 + len, r1);
-      if (((lo | hi) & 3) == 0 && ((b0 - r0) & 3) == 0) {
-        // whole 32-bit words (block starts are 32-byte aligned)
-        uint32_t* words = reinterpret_cast<uint32_t*>(bytes);
-        for (uint64_t b = lo; b < hi; b += 4) words[(b - r0) >> 2] = x[(b - b0) >> 2];
-      } else {
-        for (uint64_t b = lo; b < hi; ++b) {
-          const uint32_t w = x[(b - b0) >> 2];
-          bytes[b - r0] = (uint8_t)(w >> (8 * ((b - b0) & 3)));
-        }
-      }
-    }
-    __syncthreads();
-    for (int j = tid; j < J; j += THREADS) {
-      const uint8_t* cb = bytes + (size_t)j * B;
-      int val = 0, kk = k2;
-      while (kk > 0) {
-        if (kk >= 64) {
-          uint64_t plus = 0, minus = 0;
-#pragma unroll
-          for (int i = 0; i < 8; ++i) {
-            plus |= (uint64_t)cb[i] << (8 * i);
-            minus |= (uint64_t)cb[8 + i] << (8 * i);
-          }
-          val += __popcll(plus) - __popcll(minus);
-          cb += 16;
-          kk -= 64;
-        } else if (kk >= 8) {
-          val += __popc(cb[0]) - __popc(cb[1]);
-          cb += 2;
-          kk -= 8;
-        } else {
-          const unsigned m = (1u << kk) - 1;
-          val += __popc(cb[0] & m) - __popc(cb[1] & m);
-          break;
-        }
-      }
-      err[((size_t)p << log_n) + j0 + j] = val;
-    }
+    error_pass<THREADS>(reinterpret_cast<uint8_t*>(stage), key, e0, j0, min(per_pass, n - j0), k2,
+                        err + ((size_t)p << log_n));
     __syncthreads();
   }
+}
+
+// The sequential scan above keeps one CTA per ciphertext busy for some fifty
+// dependent passes.  Where rejections are rare (primes just below a power of
+// two: less than one expected per ciphertext) all blocks run side by side
+// instead:
+//   k_sample_guess  takes word w of the stream as output w (no rejection before
+//                   it) and records the words that its limb's prime rejects;
+//   k_sample_fix    redoes a ciphertext with 1 .. kMaxRejects of them, word w
+//                   becoming output w - (rejected words before it).  A word is
+//                   now judged by the limb it really falls in; if that ever
+//                   disagrees with the record (a shifted word at a limb boundary)
+//                   the count is set above kMaxRejects and the sequential kernel
+//                   does that ciphertext.
+// ChaCha's ALU operations bound it: 200 ciphertexts at n = 2^14, six 45-bit
+// primes take 157 us (256 us sequentially, one CTA on most SMs), 1024 take 673
+// (783), one takes 22 (164), all three launches together.
+constexpr int kGuessThreads = 256, kFixBlocks = 4;
+
+// Outputs of block g's words from `first` on, word w going to w - before(w).
+// judge(w, o, rejected) sees every word and says whether it is written.
+template <class F>
+__device__ __forceinline__ void uniform_block(const uint32_t (&key)[8], uint64_t g, int log_n,
+                                              unsigned total, int negate, uint64_t* dst,
+                                              const CtxDev& c, F&& judge) {
+  uint32_t x[16];
+  chacha_block(key, (uint32_t)(g & 127), g >> 7, x);
+  const unsigned w0 = (unsigned)word0(g);
+  const int nw = (g & 127) == 127 ? 4 : 8;
+#pragma unroll
+  for (int h = 0; h < 8; h += 2) {
+    if (h >= nw) break;
+    uint64_t v[2];
+    unsigned o[2];
+    bool put[2];
+#pragma unroll
+    for (int t = 0; t < 2; ++t) {
+      const int k = h + t;
+      o[t] = judge.index(w0 + k);
+      const PrimeDev& P = c.primes[min(o[t], total - 1) >> log_n];
+      const uint64_t q = P.q;
+      const uint64_t raw = ((uint64_t)x[2 * k + 1] << 32 | x[2 * k]) & ((1ull << P.log_q) - 1);
+      put[t] = judge(w0 + k, o[t] < total, raw >= q) && o[t] < total;
+      v[t] = negate ? q - raw : raw;
+    }
+    if (put[0] && put[1] && o[1] == o[0] + 1 && (o[0] & 1) == 0) {
+      *reinterpret_cast<ulonglong2*>(dst + o[0]) = make_ulonglong2(v[0], v[1]);
+    } else {
+      if (put[0]) dst[o[0]] = v[0];
+      if (put[1]) dst[o[1]] = v[1];
+    }
+  }
+}
+
+struct GuessJudge {
+  Rejects* r;
+  __device__ __forceinline__ unsigned index(unsigned w) const { return w; }
+  __device__ __forceinline__ bool operator()(unsigned w, bool inside, bool rejected) const {
+    if (inside && rejected) {
+      const unsigned i = atomicAdd(&r->count, 1u);
+      if (i < kMaxRejects) r->word[i] = w;
+    }
+    return true;
+  }
+};
+
+// grid (uniform CTAs + error CTAs, ciphertexts)
+__global__ void __launch_bounds__(kGuessThreads)
+    k_sample_guess(uint64_t* a_dst, size_t a_stride, int negate, int32_t* err,
+                   const uint8_t* seeds, int L, int variance, int log_n, int uniform_ctas,
+                   Rejects* rejects, CtxDev c) {
+  __shared__ uint8_t bytes[kGuessThreads * 64];
+  const int p = blockIdx.y, n = 1 << log_n;
+  const unsigned total = (unsigned)L << log_n;
+  uint32_t key[8];
+  load_seed(seeds, p, key);
+  if ((int)blockIdx.x >= uniform_ctas) {
+    const int k2 = 2 * variance, per_pass = error_per_pass<kGuessThreads>(k2);
+    const int j0 = ((int)blockIdx.x - uniform_ctas) * per_pass;
+    error_pass<kGuessThreads>(bytes, key, (uint64_t)total * 8, j0, min(per_pass, n - j0), k2,
+                              err + ((size_t)p << log_n));
+    return;
+  }
+  const uint64_t g = (uint64_t)blockIdx.x * kGuessThreads + threadIdx.x;
+  if (word0(g) < total)
+    uniform_block(key, g, log_n, total, negate, a_dst + (size_t)p * a_stride, c,
+                  GuessJudge{rejects + p});
+}
+
+struct FixJudge {
+  const Rejects* r;
+  unsigned n;
+  bool* hard;
+  __device__ __forceinline__ unsigned index(unsigned w) const {
+    unsigned before = 0;
+    for (unsigned i = 0; i < n; ++i) before += r->word[i] < w;
+    return w - before;
+  }
+  __device__ __forceinline__ bool operator()(unsigned w, bool inside, bool rejected) const {
+    bool listed = false;
+    for (unsigned i = 0; i < n; ++i) listed |= r->word[i] == w;
+    if (inside && listed != rejected) *hard = true;
+    return !listed;
+  }
+};
+
+__global__ void __launch_bounds__(kGuessThreads)
+    k_sample_fix(uint64_t* a_dst, size_t a_stride, int negate, int32_t* err,
+                 const uint8_t* seeds, int L, int variance, int log_n, int uniform_ctas,
+                 Rejects* rejects, CtxDev c) {
+  __shared__ uint8_t bytes[kGuessThreads * 64];
+  __shared__ Rejects rec;
+  const int p = blockIdx.y, n = 1 << log_n;
+  // Another CTA of this ciphertext may raise the count meanwhile; then what this
+  // one does or leaves out is redone anyway.
+  if (threadIdx.x == 0) {
+    rec.count = *(volatile unsigned*)&rejects[p].count;
+    for (unsigned i = 0; i < kMaxRejects; ++i) rec.word[i] = rejects[p].word[i];
+  }
+  __syncthreads();
+  const unsigned found = rec.count;
+  if (found == 0 || found > kMaxRejects) return;
+  const unsigned total = (unsigned)L << log_n;
+  uint32_t key[8];
+  load_seed(seeds, p, key);
+  if ((int)blockIdx.x >= uniform_ctas) {
+    const int k2 = 2 * variance, per_pass = error_per_pass<kGuessThreads>(k2);
+    for (int i = 0; i < kFixBlocks; ++i) {
+      const int j0 = (((int)blockIdx.x - uniform_ctas) * kFixBlocks + i) * per_pass;
+      if (j0 >= n) break;
+      error_pass<kGuessThreads>(bytes, key, ((uint64_t)total + found) * 8, j0,
+                                min(per_pass, n - j0), k2, err + ((size_t)p << log_n));
+      __syncthreads();
+    }
+    return;
+  }
+  bool hard = false;
+  for (int i = 0; i < kFixBlocks; ++i) {
+    const uint64_t g = ((uint64_t)blockIdx.x * kFixBlocks + i) * kGuessThreads + threadIdx.x;
+    if (word0(g) < (uint64_t)total + found)
+      uniform_block(key, g, log_n, total, negate, a_dst + (size_t)p * a_stride, c,
+                    FixJudge{&rec, found, &hard});
+  }
+  if (hard) atomicMax(&rejects[p].count, kMaxRejects + 1);
 }
 
 // Signed error e (|e| < q) as the Montgomery value of e mod q: the balanced
@@ -295,18 +464,40 @@ __global__ void k_bgv_enc_combine(uint64_t* out, const uint64_t* e_ntt, const ui
 
 }  // namespace
 
+size_t sample_reject_bytes() { return sizeof(Rejects); }
+
 int sample_error_bytes(int variance) { return error_bytes(2 * variance); }
 
 void launch_sample_uniform_error(const CtxDev& c, uint64_t* a_dst, size_t a_stride,
                                  int negate, int32_t* err, const uint8_t* seeds, int L,
-                                 int variance, int count, cudaStream_t s) {
+                                 int variance, int count, void* rejects, cudaStream_t s) {
   if (count <= 0) return;
   LaunchScope scope_("sample_uniform_error", s);
   // 256-thread CTAs: four per SM (64 registers each), so 1024 ciphertexts
   // take 1.7 waves of 608 slots rather than 3.4 waves of 304.
   constexpr int T = 256;
+  Rejects* r = reinterpret_cast<Rejects*>(rejects);
+  if (r) {
+    g_launch_count += 2;
+    const auto ceil = [](long long a, long long b) { return (int)((a + b - 1) / b); };
+    const long long total = (long long)L << c.log_n;
+    const int ectas = ceil(c.n, error_per_pass<kGuessThreads>(2 * variance));
+    const int uctas = ceil(block_of_word(total - 1) + 1, kGuessThreads);
+    const int fctas = ceil(block_of_word(total + kMaxRejects) + 1, kGuessThreads * kFixBlocks);
+    cudaMemsetAsync(r, 0, sizeof(Rejects) * count, s);
+    for (int p0 = 0; p0 < count; p0 += 65535) {
+      const int pc = std::min(count - p0, 65535);
+      uint64_t* a = a_dst + (size_t)p0 * a_stride;
+      int32_t* e = err + ((size_t)p0 << c.log_n);
+      const uint8_t* sd = seeds + (size_t)p0 * 32;
+      k_sample_guess<<<dim3(uctas + ectas, pc), kGuessThreads, 0, s>>>(
+          a, a_stride, negate, e, sd, L, variance, c.log_n, uctas, r + p0, c);
+      k_sample_fix<<<dim3(fctas + ceil(ectas, kFixBlocks), pc), kGuessThreads, 0, s>>>(
+          a, a_stride, negate, e, sd, L, variance, c.log_n, fctas, r + p0, c);
+    }
+  }
   k_sample_uniform_error<T><<<count, T, 0, s>>>(a_dst, a_stride, negate, err, seeds, L,
-                                                variance, c.log_n, c);
+                                                variance, c.log_n, r, c);
 }
 
 void launch_error_lift(const CtxDev& c, uint64_t* out, const int32_t* err, int count, int L,
