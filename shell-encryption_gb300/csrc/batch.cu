@@ -462,12 +462,16 @@ int shg_batch_autotune(shg_batch* b, int reps, shg_stream stream) {
       return r;
     };
     // Transform organisation: one CTA per limb or the four-step kernels.
+    // (13, the default, means 12 but for ModReduce.)
+    auto four_step_from = [&](const Tuning& t) {
+      return t.four_step_min == 13 && g.gk.kind != SHG_OP_MODREDUCE ? 12 : t.four_step_min;
+    };
     if (g.log_n >= 12 && g.log_n <= 14) {
       Tuning c = best;
-      c.four_step_min = best.four_step_min <= g.log_n ? 16 : g.log_n;
+      c.four_step_min = four_step_from(best) <= g.log_n ? 16 : g.log_n;
       if ((st = consider(c))) break;
     }
-    const bool four_step = g.log_n >= best.four_step_min || g.log_n > 14;
+    const bool four_step = g.log_n >= four_step_from(best) || g.log_n > 14;
     if (g.gk.kind != SHG_OP_MODREDUCE) {
       if (four_step && g.log_n >= 12) {
         Tuning c = best;

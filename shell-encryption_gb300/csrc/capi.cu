@@ -4,6 +4,7 @@
 #include <cuda_runtime.h>
 
 #include <algorithm>
+#include <climits>
 #include <cmath>
 #include <cstdlib>
 #include <cstdio>
@@ -181,8 +182,7 @@ struct shg_context {
   int chunk_cts = 0;
   int small_q = 0;  // all moduli below 2^58
   int narrow_q = 0;  // all moduli below 2^45
-  int ntt4_min = 13;  // four-step transforms from this log_n up (measured faster
-                      // for every operation from n = 2^13; mixed at 2^12)
+  int ntt4_min = 13;  // four-step transforms from this log_n up (see key_min())
   int ntt4_plain_min = 12;  // plain forward / inverse NTTs: four-step from 2^12
                             // (8-10 % faster there) unless the threshold is set
                             // above 13
@@ -216,16 +216,22 @@ struct shg_context {
     shg::Crt32* d_crt = nullptr;
   } set32[2];
 
+  // At the default threshold (13) key switches, products and encryption take the
+  // four-step kernels from n = 2^12 as plain NTTs do, ModReduce from 2^13 (n = 2^12,
+  // 256 ciphertexts, one CTA per limb against four-step: products of 1 / 2 / 3
+  // limbs 184 / 298 / 448 against 146 / 235 / 351 us, rotations of 3 limbs 477 /
+  // 409, encryptions 120 / 100, ModReduce of 6 limbs 146 / 157).
+  int key_min() const { return ntt4_min == 13 ? 12 : ntt4_min; }
   CtxDev dev() const {
-    return CtxDev{log_n, n, L, d_primes, d_tw_fwd, d_tw_inv, d_qmod, small_q, ntt4_min,
-                  ks_fused, sms, ntt4_plain_min, narrow_q};
+    return CtxDev{log_n, n, L, d_primes, d_tw_fwd, d_tw_inv, d_qmod, small_q, key_min(),
+                  ks_fused, sms, ntt4_plain_min, ntt4_min, narrow_q};
   }
   // The auxiliary primes as a context of their own (NTTs and pointwise ops
   // over aux limbs); there is no cross-prime table in this view.
   CtxDev aux_dev() const {
     return CtxDev{log_n, n, K, d_primes + L, d_tw_fwd + (size_t)L * n,
-                  d_tw_inv + (size_t)L * n, nullptr, small_q, ntt4_min, ks_fused, sms,
-                  ntt4_plain_min, narrow_q};
+                  d_tw_inv + (size_t)L * n, nullptr, small_q, key_min(), ks_fused, sms,
+                  ntt4_plain_min, ntt4_min, narrow_q};
   }
   int ensure_ws(size_t bytes) {
     if (bytes <= ws_bytes) return SHG_OK;
@@ -328,14 +334,19 @@ size_t ks_scratch_bytes(const shg_context* ctx, const shg_key* key, const shg::K
   return (size_t)key->k * key->L * ctx->n * sizeof(uint64_t);
 }
 
-// Cts per pipeline chunk, bounded by the scratch budget.
-int chunk_for(shg_context* ctx, size_t per_ct_bytes, int count) {
-  int c = ctx->chunk_cts > 0 ? ctx->chunk_cts : 16;
-  const size_t budget = (size_t)1 << 30;  // 1 GiB default scratch ceiling
-  const size_t cap = std::max<size_t>(1, budget / std::max<size_t>(per_ct_bytes, 1));
-  if ((size_t)c > cap) c = (int)cap;
-  if (c > count) c = count;
-  return std::max(c, 1);
+// Ciphertexts per chunk of a batched key switch with per_ct bytes of scratch
+// each: the context's setting (at most set_max), or 16 where they have megabytes
+// (n = 2^14, six limbs: 4, 8, 12, 16 take 3175, 2689, 2615, 2595 us for 256
+// products), as many as fit 48 MB, still two chunks for the two lanes, where less
+// (16 / 32 / 64 per chunk, 256 products: n = 2^12, two limbs 235 / 198 / 174 us,
+// n = 2^13, three limbs 611 / 571 / 567, n = 2^11, six limbs 733 / 744 / 754); at
+// most `budget` bytes.
+int ks_chunk(const shg_context* ctx, size_t per_ct, int count, size_t budget, int set_max) {
+  const int most = (int)std::max<size_t>(1, budget / std::max<size_t>(per_ct, 1));
+  if (ctx->chunk_cts > 0)
+    return std::max(1, std::min({ctx->chunk_cts, set_max, set_max > 16 ? most : 16, count}));
+  const int small = (int)std::min<size_t>((count + 1) / 2, ((size_t)48 << 20) / per_ct);
+  return std::max(1, std::min({std::max(16, small), most, count}));
 }
 
 // ---- RNS basis conversion tables (BFV) --------------------------------------
@@ -1190,14 +1201,15 @@ struct KsLanes {
   int n = 1;
   // At most `want` lanes (and the context's setting).
   int open(int want) {
-    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-    SHG_CUDA(cudaStreamIsCapturing(s, &cap));
-    if (!ctx->ks_fork && std::min(want, ctx->ks_lanes) > 1 &&
-        cap == cudaStreamCaptureStatusNone) {
-      SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_fork, cudaEventDisableTiming));
-      for (int i = 0; i < shg_context::kMaxKsLanes - 1; ++i) {
-        SHG_CUDA(cudaStreamCreateWithFlags(&ctx->ks_side[i], cudaStreamNonBlocking));
-        SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_join[i], cudaEventDisableTiming));
+    if (!ctx->ks_fork && std::min(want, ctx->ks_lanes) > 1) {
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      SHG_CUDA(cudaStreamIsCapturing(s, &cap));
+      if (cap == cudaStreamCaptureStatusNone) {
+        for (int i = 0; i < shg_context::kMaxKsLanes - 1; ++i) {
+          SHG_CUDA(cudaStreamCreateWithFlags(&ctx->ks_side[i], cudaStreamNonBlocking));
+          SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_join[i], cudaEventDisableTiming));
+        }
+        SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_fork, cudaEventDisableTiming));
       }
     }
     n = lanes_of(want);
@@ -1236,8 +1248,9 @@ int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
   const size_t per_ct = Ln * sizeof(uint64_t) + d_per_ct;
   const size_t per_ct_plain =
       Ln * sizeof(uint64_t) + ks_scratch_bytes(ctx, key, shg::Ks32{});
-  const int C = chunk_for(ctx, per_ct, count);
-  const int C_plain = chunk_for(ctx, per_ct_plain, count);
+  constexpr size_t kBudget = (size_t)1 << 30;
+  const int C = ks_chunk(ctx, per_ct, count, kBudget, INT_MAX);
+  const int C_plain = ks_chunk(ctx, per_ct_plain, count, kBudget, INT_MAX);
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
   std::lock_guard<std::mutex> lock(ctx->mu);
   // Each lane has its own X and D; two chunks side by side measured 17 % faster
@@ -1335,12 +1348,8 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
   const size_t x_bytes = (size_t)count * Ln * sizeof(uint64_t);
   const shg::Ks32& ks32 = ks32_for(ctx, key, count, keys == nullptr);
   const size_t d_per_ct = ks_scratch_bytes(ctx, key, ks32);
-  // 16 ciphertexts per chunk measured fastest at n = 2^14, L = 6 (the digit
-  // kernel's grid is then ~13.8 K CTAs).
   auto chunk_of = [&](size_t per_ct) {
-    int c = ctx->chunk_cts > 0 ? ctx->chunk_cts
-                               : (int)std::max<size_t>(1, ((size_t)256 << 20) / per_ct);
-    return std::max(1, std::min({c, 16, count}));
+    return ks_chunk(ctx, per_ct, count, (size_t)256 << 20, 16);
   };
   const int C = chunk_of(d_per_ct);
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
@@ -1451,9 +1460,7 @@ int mul_relin_host_impl(shg_context* ctx, const shg_key* key, void* out_v, const
   const shg::Ks32& ks32 = ks32_for(ctx, key, count, true);
   const size_t d_per_ct = ks_scratch_bytes(ctx, key, ks32);
   auto chunk_of = [&](size_t per_ct) {
-    int c = ctx->chunk_cts > 0 ? ctx->chunk_cts
-                               : (int)std::max<size_t>(1, ((size_t)256 << 20) / per_ct);
-    return std::max(1, std::min({c, 16, P}));
+    return ks_chunk(ctx, per_ct, P, (size_t)256 << 20, 16);
   };
   const int C = chunk_of(d_per_ct);
   const size_t d_plain = ks_scratch_bytes(ctx, key, shg::Ks32{});
@@ -2390,7 +2397,7 @@ int shg_bgv_encrypt(shg_context* ctx, uint64_t* out, const uint64_t* key,
   const size_t n = ctx->n, Ln = (size_t)L * n;
   shg::ScalarPack tm{};
   for (int l = 0; l < L; ++l) tm.v[l] = to_mont(ctx->t % ctx->hp[l].q, ctx->hp[l].q);
-  const bool four = ctx->log_n >= 12 && (ctx->log_n >= ctx->ntt4_min || ctx->log_n > 14);
+  const bool four = ctx->log_n >= 12 && (ctx->log_n >= ctx->key_min() || ctx->log_n > 14);
   // Transform chunks as large as 1 GiB of scratch allows (or the context's
   // chunk setting): whole-batch launches measured faster (n = 2^14, six
   // limbs, 1024 ciphertexts: 1.50 ms) than L2-sized 42-ciphertext chunks

@@ -1046,6 +1046,7 @@ namespace {
 // Transforms of n >= 2^ntt4_min (always n = 2^15) run as two four-step
 // phase kernels (ntt4.cu); smaller ones as one CTA-resident kernel.
 bool use_ntt4(const CtxDev& c) { return c.log_n >= c.ntt4_min || c.log_n > 14; }
+bool use_ntt4_mod(const CtxDev& c) { return c.log_n >= c.ntt4_mod_min || c.log_n > 14; }
 bool use_ntt4_plain(const CtxDev& c) {
   return c.log_n >= 12 && (c.log_n >= c.ntt4_plain_min || c.log_n > 14);
 }
@@ -1077,14 +1078,15 @@ void launch_ntt_fwd(const CtxDev& c, const uint64_t* in, uint64_t* out, int num,
 #undef F
 }
 
-// plain: a plain inverse NTT call (the plain-NTT threshold applies).
+// plain: a plain inverse NTT call (the plain-NTT threshold applies; else
+// ModReduce's).
 static void launch_ntt_inv_scaled(const CtxDev& c, const uint64_t* in,
                                   uint64_t* out, int num, int L, int in_first,
                                   int in_stride, int mode, uint64_t sw,
                                   uint64_t swp, cudaStream_t s, bool plain = false) {
   if (num <= 0) return;
   LaunchScope scope_("ntt_inv", s);
-  if (plain ? use_ntt4_plain(c) : use_ntt4(c)) {
+  if (plain ? use_ntt4_plain(c) : use_ntt4_mod(c)) {
     g_launch_count++;  // second phase kernel
     launch4_ntt_inv(c, in, out, num, L, in_first, in_stride, mode, sw, swp, s);
     return;
@@ -1269,7 +1271,7 @@ void launch_modreduce_ntt(const CtxDev& c, uint64_t* out, uint64_t* Y,
   launch_ntt_inv_scaled(c, in, Y, count, L, L - 1, L, 2, k_plain, k_shoup, s);
   // Stage 2: lift, forward NTT, combine.
   LaunchScope scope_("modreduce_lift", s);
-  if (use_ntt4(c)) {
+  if (use_ntt4_mod(c)) {
     g_launch_count++;  // second phase kernel
     launch4_modreduce_lift(c, out, Y, in, sc, count, L, s);
     return;
