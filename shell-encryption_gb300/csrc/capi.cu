@@ -181,6 +181,7 @@ struct shg_context {
   size_t ws_bytes = 0;
   int chunk_cts = 0;
   int small_q = 0;  // all moduli below 2^58
+  int lazy_inv = 0;  // all moduli below 2^53
   int narrow_q = 0;  // all moduli below 2^45
   int ntt4_min = 13;  // four-step transforms from this log_n up (see key_min())
   int ntt4_plain_min = 12;  // plain forward / inverse NTTs: four-step from 2^12
@@ -224,14 +225,14 @@ struct shg_context {
   int key_min() const { return ntt4_min == 13 ? 12 : ntt4_min; }
   CtxDev dev() const {
     return CtxDev{log_n, n, L, d_primes, d_tw_fwd, d_tw_inv, d_qmod, small_q, key_min(),
-                  ks_fused, sms, ntt4_plain_min, ntt4_min, narrow_q};
+                  ks_fused, sms, ntt4_plain_min, ntt4_min, narrow_q, lazy_inv};
   }
   // The auxiliary primes as a context of their own (NTTs and pointwise ops
   // over aux limbs); there is no cross-prime table in this view.
   CtxDev aux_dev() const {
     return CtxDev{log_n, n, K, d_primes + L, d_tw_fwd + (size_t)L * n,
                   d_tw_inv + (size_t)L * n, nullptr, small_q, key_min(), ks_fused, sms,
-                  ntt4_plain_min, ntt4_min, narrow_q};
+                  ntt4_plain_min, ntt4_min, narrow_q, lazy_inv};
   }
   int ensure_ws(size_t bytes) {
     if (bytes <= ws_bytes) return SHG_OK;
@@ -348,6 +349,51 @@ int ks_chunk(const shg_context* ctx, size_t per_ct, int count, size_t budget, in
   const int small = (int)std::min<size_t>((count + 1) / 2, ((size_t)48 << 20) / per_ct);
   return std::max(1, std::min({std::max(16, small), most, count}));
 }
+
+// Streams that the independent parts of one batched call rotate over: lane 0 is
+// the caller's, the others the context's (made outside any stream capture, by
+// the first call that wants them; without them there is one lane).  Parts on
+// other lanes fill the tails of each other's launches.  Under ctx->mu.
+struct KsLanes {
+  shg_context* ctx;
+  cudaStream_t s;
+  int n = 1;
+  // At most `want` lanes (and the context's setting).
+  int open(int want) {
+    if (!ctx->ks_fork && std::min(want, ctx->ks_lanes) > 1) {
+      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+      SHG_CUDA(cudaStreamIsCapturing(s, &cap));
+      if (cap == cudaStreamCaptureStatusNone) {
+        for (int i = 0; i < shg_context::kMaxKsLanes - 1; ++i) {
+          SHG_CUDA(cudaStreamCreateWithFlags(&ctx->ks_side[i], cudaStreamNonBlocking));
+          SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_join[i], cudaEventDisableTiming));
+        }
+        SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_fork, cudaEventDisableTiming));
+      }
+    }
+    n = lanes_of(want);
+    return SHG_OK;
+  }
+  int lanes_of(int want) const {
+    return ctx->ks_fork ? std::max(1, std::min(ctx->ks_lanes, want)) : 1;
+  }
+  cudaStream_t stream(int lane) const { return lane ? ctx->ks_side[lane - 1] : s; }
+  // The side lanes start after what is on lane 0 now; lane 0 goes on after them.
+  int fork() const {
+    if (n == 1) return SHG_OK;
+    SHG_CUDA(cudaEventRecord(ctx->ks_fork, s));
+    for (int i = 0; i + 1 < n; ++i)
+      SHG_CUDA(cudaStreamWaitEvent(ctx->ks_side[i], ctx->ks_fork, 0));
+    return SHG_OK;
+  }
+  int join() const {
+    for (int i = 0; i + 1 < n; ++i) {
+      SHG_CUDA(cudaEventRecord(ctx->ks_join[i], ctx->ks_side[i]));
+      SHG_CUDA(cudaStreamWaitEvent(s, ctx->ks_join[i], 0));
+    }
+    return SHG_OK;
+  }
+};
 
 // ---- RNS basis conversion tables (BFV) --------------------------------------
 //
@@ -534,15 +580,19 @@ int shg_context_create_with_aux(int log_n, const uint64_t* qs, int num_qs, const
     d.half_q = h.q >> 1;
     d.log_q = (uint64_t)h.log_q;
     d.barrett = h.barrett_num;
+    d.red_shift = (uint32_t)std::max(h.log_q - 16, 0);
+    d.red_mul = (uint32_t)(((u128)1 << (32 + d.red_shift)) / h.q);
     for (int j = 0; j < n; ++j) {
       twf[(size_t)i * n + j] = Tw{h.fwd[j], shoup_of(h.fwd[j], h.q)};
       twi[(size_t)i * n + j] = Tw{h.inv[j], shoup_of(h.inv[j], h.q)};
     }
   }
   ctx->small_q = 1;
+  ctx->lazy_inv = 1;
   ctx->narrow_q = 1;
   for (int i = 0; i < NP; ++i) {
     if ((all[i] >> 58) != 0) ctx->small_q = 0;
+    if ((all[i] >> 53) != 0) ctx->lazy_inv = 0;
     if ((all[i] >> 45) != 0) ctx->narrow_q = 0;
   }
   ctx->qmod.resize((size_t)L * L);
@@ -1190,51 +1240,6 @@ struct KsArgs {
 
 int upload_key_table(const shg_key* const* keys, int count, int stride, int offset,
                      const uint64_t** dst, shg::KeyTable* out, cudaStream_t s);
-
-// Streams that the independent parts of one batched call rotate over: lane 0 is
-// the caller's, the others the context's (made outside any stream capture, by
-// the first call that wants them; without them there is one lane).  Parts on
-// other lanes fill the tails of each other's launches.  Under ctx->mu.
-struct KsLanes {
-  shg_context* ctx;
-  cudaStream_t s;
-  int n = 1;
-  // At most `want` lanes (and the context's setting).
-  int open(int want) {
-    if (!ctx->ks_fork && std::min(want, ctx->ks_lanes) > 1) {
-      cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
-      SHG_CUDA(cudaStreamIsCapturing(s, &cap));
-      if (cap == cudaStreamCaptureStatusNone) {
-        for (int i = 0; i < shg_context::kMaxKsLanes - 1; ++i) {
-          SHG_CUDA(cudaStreamCreateWithFlags(&ctx->ks_side[i], cudaStreamNonBlocking));
-          SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_join[i], cudaEventDisableTiming));
-        }
-        SHG_CUDA(cudaEventCreateWithFlags(&ctx->ks_fork, cudaEventDisableTiming));
-      }
-    }
-    n = lanes_of(want);
-    return SHG_OK;
-  }
-  int lanes_of(int want) const {
-    return ctx->ks_fork ? std::max(1, std::min(ctx->ks_lanes, want)) : 1;
-  }
-  cudaStream_t stream(int lane) const { return lane ? ctx->ks_side[lane - 1] : s; }
-  // The side lanes start after what is on lane 0 now; lane 0 goes on after them.
-  int fork() const {
-    if (n == 1) return SHG_OK;
-    SHG_CUDA(cudaEventRecord(ctx->ks_fork, s));
-    for (int i = 0; i + 1 < n; ++i)
-      SHG_CUDA(cudaStreamWaitEvent(ctx->ks_side[i], ctx->ks_fork, 0));
-    return SHG_OK;
-  }
-  int join() const {
-    for (int i = 0; i + 1 < n; ++i) {
-      SHG_CUDA(cudaEventRecord(ctx->ks_join[i], ctx->ks_side[i]));
-      SHG_CUDA(cudaStreamWaitEvent(s, ctx->ks_join[i], 0));
-    }
-    return SHG_OK;
-  }
-};
 
 // Gadget key switch of component a.comp of `count` ciphertexts; with `keys`,
 // member i uses keys[i] (same gadget shape as `key`).

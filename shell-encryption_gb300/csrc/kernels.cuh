@@ -37,6 +37,8 @@ struct CtxDev {
   int ntt4_plain_min;         // the same threshold for plain forward / inverse NTTs
   int ntt4_mod_min;           // and for ModReduce
   int narrow_q;               // every q below 2^45 (implies small_q)
+  int lazy_inv;               // every q below 2^53 (implies small_q): four-step inverse phases
+                              // skip their conditional subtractions
 };
 
 // Per-digit description of a gadget key (RnsGadget::Decompose order,

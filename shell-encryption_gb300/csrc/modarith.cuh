@@ -26,7 +26,9 @@ struct PrimeDev {
   uint64_t half_q;         // floor(q / 2): balanced-lift threshold
   uint64_t log_q;
   uint64_t barrett;        // floor(2^64 / q): x mod q for any 64-bit x
-  uint64_t pad[2];
+  uint32_t red_mul;        // floor(2^(32 + red_shift) / q), for reduce_1024
+  uint32_t red_shift;      // max(log_q - 16, 0)
+  uint64_t pad;
 };
 static_assert(sizeof(PrimeDev) == 128, "PrimeDev is one cache line");
 
@@ -176,6 +178,15 @@ __device__ __forceinline__ uint64_t reduce_4q(uint64_t x, uint64_t q,
                                               uint64_t two_q) {
   x = x >= two_q ? x - two_q : x;
   return x >= q ? x - q : x;
+}
+
+// x mod q in [0, 2q) for x below 2^10 q (and 2^64): the quotient (at most 10
+// bits) from the top bits of x, at most one too small: the shifted-out part of x
+// is below 2^-15 q and the rounding of mul costs x / 2^(32 + shift) < 2^-6.  Four
+// instructions where the Barrett product by floor(2^64 / q) takes some twenty.
+__device__ __forceinline__ uint64_t reduce_1024(uint64_t x, uint64_t q, uint32_t mul,
+                                                uint32_t shift) {
+  return x + (uint64_t)__umulhi((uint32_t)(x >> shift), mul) * (0 - q);
 }
 
 __device__ __forceinline__ uint64_t shoup(uint64_t x, uint64_t w, uint64_t wp,

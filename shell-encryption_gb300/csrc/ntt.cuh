@@ -122,6 +122,20 @@ __device__ __forceinline__ void bf_gs(uint64_t& X, uint64_t& Y, Tw w,
   }
 }
 
+// Gentleman-Sande butterfly of level V of a phase without any correction, for
+// primes below 2^53: inputs below 2^(2 + V) q, the sum below twice that, the
+// product below 4q.  At most eight levels: differences stay below 2^11 q < 2^64.
+template <int V>
+__device__ __forceinline__ void bf_gs_lazy(uint64_t& X, uint64_t& Y, Tw w, uint64_t q) {
+  const uint64_t d = X - Y + (q << (2 + V));
+  X = X + Y;
+  Y = shoup_lazy4(d, w.w, w.wp, q);
+}
+
+// Inverse butterflies: kInvExact and kInvWide are bf_gs's two, kInvLazy
+// bf_gs_lazy.
+enum : int { kInvExact = 0, kInvWide = 1, kInvLazy = 2 };
+
 // Coefficients per thread: 16, or 32 at n = 2^14 (512 threads, so a thread
 // may use 128 registers and the transform needs one exchange less).
 __host__ __device__ constexpr int default_elog(int log_n) {
@@ -231,7 +245,7 @@ struct NttCore {
   // transform (bit_off = 0, row = 0), for row r of a transform whose low
   // LOG_N bits form the rows (bit_off = 0, row = r), and for the columns of
   // one whose low bit_off bits were done first (row = 0).
-  template <int p, bool WIDE = false>
+  template <int p, int INV = kInvExact>
   __device__ __forceinline__ static void inv_pass(uint64_t (&x)[E], int tid,
                                                   const Tw* __restrict__ tw,
                                                   int nfull, int bit_off,
@@ -252,7 +266,10 @@ struct NttCore {
         static_for<0, (1 << lb)>([&](auto ll) {
           constexpr int k0 = (u << (lb + 1)) | decltype(ll)::value;
           constexpr int k1 = k0 | (1 << lb);
-          bf_gs<WIDE>(x[k0], x[k1], w, q, two_q);
+          if constexpr (INV == kInvLazy)
+            bf_gs_lazy<b>(x[k0], x[k1], w, q);
+          else
+            bf_gs<INV == kInvWide>(x[k0], x[k1], w, q, two_q);
         });
       });
     });
@@ -310,11 +327,12 @@ struct NttCore {
 
   // Full inverse transform without the n^{-1} scaling (input in inv_in
   // layout, values in [0, 2q); output in inv_out layout, values in [0, 2q);
-  // WIDE: [0, 4q) both, for primes below 2^58).  Every caller finishes with
+  // kInvWide: [0, 4q) both, for primes below 2^58; kInvLazy, below 2^53: input in
+  // [0, 4q), sums of the last level below 2^(2 + LOG_N) q, products below 4q).  Every caller finishes with
   // an exact Shoup product (the n^{-1} scaling), which takes any 64-bit value;
   // a caller that stores the output without that product must reduce it
-  // (below 4q with WIDE, below 2q otherwise).
-  template <bool WIDE = false, class Map = SwzMap>
+  // (to the ranges above).
+  template <int INV = kInvExact, class Map = SwzMap>
   __device__ __forceinline__ static void inverse_m(uint64_t (&x)[E], int tid,
                                                    const Map& m,
                                                    const Tw* __restrict__ tw,
@@ -323,17 +341,17 @@ struct NttCore {
                                                    uint64_t two_q) {
     static_for<0, P>([&](auto pp) {
       constexpr int p = decltype(pp)::value;
-      inv_pass<p, WIDE>(x, tid, tw, nfull, bit_off, row, q, two_q);
+      inv_pass<p, INV>(x, tid, tw, nfull, bit_off, row, q, two_q);
       if constexpr (p + 1 < P) exchange(x, tid, m, inv_clo(p), inv_clo(p + 1));
     });
   }
-  template <bool WIDE = false>
+  template <int INV = kInvExact>
   __device__ __forceinline__ static void inverse(uint64_t (&x)[E], int tid,
                                                  uint64_t* sm,
                                                  const Tw* __restrict__ tw,
                                                  int nfull, int row, uint64_t q,
                                                  uint64_t two_q) {
-    inverse_m<WIDE>(x, tid, SwzMap{sm}, tw, nfull, 0, row, q, two_q);
+    inverse_m<INV>(x, tid, SwzMap{sm}, tw, nfull, 0, row, q, two_q);
   }
 };
 

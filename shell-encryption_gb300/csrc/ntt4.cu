@@ -133,8 +133,9 @@ struct FwdSrcError {
 };
 
 // ---------------------------------------------------------------------------
-// Forward phase-2 sinks: the values at i, i + 1 of transform g -- canonical,
-// or below 62 q (lazy, small primes) for sinks with kTakesLazy.
+// Forward phase-2 sinks: the values at i, i + 1 of transform g = l + L m (its
+// limb l, L of pm) -- canonical, or below 62 q (lazy, small primes) for sinks
+// with kTakesLazy.
 // ---------------------------------------------------------------------------
 
 template <int LOG_N>
@@ -147,8 +148,8 @@ struct FwdDstPlain {
       *reinterpret_cast<ulonglong2*>(base + i) = make_ulonglong2(x0, x1);
     }
   };
-  __device__ H bind(int g, int, const CtxDev&) const { return H{p + ((size_t)g << LOG_N)}; }
-  __device__ void prefetch(int, int, int) const {}
+  __device__ H bind(int, int g, int, const CtxDev&) const { return H{p + ((size_t)g << LOG_N)}; }
+  __device__ void prefetch(int, int, int, int) const {}
 };
 
 // ModReduceLsb combine: out_i = in_i * c1 + delta_i * c2
@@ -174,9 +175,7 @@ struct FwdDstModCombine {
       *reinterpret_cast<ulonglong2*>(o + i) = r;
     }
   };
-  __device__ H bind(int g, int i, const CtxDev& c) const {
-    const int Lr = L - 1;
-    const int p = g / Lr;
+  __device__ H bind(int p, int g, int i, const CtxDev& c) const {
     H h;
     h.o = out + ((size_t)g << LOG_N);
     h.a = in + (((size_t)p * L + i) << LOG_N);
@@ -188,8 +187,8 @@ struct FwdDstModCombine {
     return h;
   }
   // The 16 values of limb i of `in` that the sink reads at i0.
-  __device__ void prefetch(int g, int i, int i0) const {
-    prefetch_l2(in + ((((size_t)(g / (L - 1)) * L + i) << LOG_N) + i0));
+  __device__ void prefetch(int p, int, int i, int i0) const {
+    prefetch_l2(in + (((size_t)p * L + i) << LOG_N) + i0);
   }
 };
 
@@ -223,8 +222,7 @@ struct FwdDstBgvEnc {
       *reinterpret_cast<ulonglong2*>(o + i) = r;
     }
   };
-  __device__ H bind(int g, int i, const CtxDev& c) const {
-    const int p = g / L;
+  __device__ H bind(int p, int g, int i, const CtxDev& c) const {
     H h;
     h.o = out + (((size_t)p * 2 * L + i) << LOG_N);
     h.mm = m + ((size_t)g << LOG_N);
@@ -237,9 +235,9 @@ struct FwdDstBgvEnc {
   }
   // Plaintext and c1 lines the sink reads at i0, fetched while the row
   // transform runs.
-  __device__ void prefetch(int g, int i, int i0) const {
+  __device__ void prefetch(int p, int g, int i, int i0) const {
     prefetch_l2(m + ((size_t)g << LOG_N) + i0);
-    prefetch_l2(out + ((((size_t)(g / L) * 2 + 1) * L + i) << LOG_N) + i0);
+    prefetch_l2(out + ((((size_t)p * 2 + 1) * L + i) << LOG_N) + i0);
   }
 };
 
@@ -276,9 +274,9 @@ struct FwdDstKsBase {
           make_ulonglong2(add_mod(v.x, x0, q), add_mod(v.y, x1, q));
     }
   };
-  __device__ H bind(int g, int l, const CtxDev& c) const {
-    const int comp = (g / L) & 1;
-    const size_t p = (size_t)(g / (2 * L));
+  __device__ H bind(int m, int g, int l, const CtxDev& c) const {
+    const int comp = m & 1;
+    const size_t p = (size_t)(m >> 1);
     H h;
     h.o = out + ((size_t)g << LOG_N);
     h.b = comp && base1_zero
@@ -288,7 +286,7 @@ struct FwdDstKsBase {
     h.q = c.primes[l].q;
     return h;
   }
-  __device__ void prefetch(int, int, int) const {}
+  __device__ void prefetch(int, int, int, int) const {}
 };
 
 // ---------------------------------------------------------------------------
@@ -493,62 +491,6 @@ __global__ void __launch_bounds__(Ntt4<LOG_N>::COL_THREADS,
     uint64_t* dst = D + (((p * k + j) * L + l) << LOG_N);
 #pragma unroll
     for (int e = 0; e < C::E; ++e) dst[(C::fwd_out_idx(t, e) << S::B) | col] = x[e];
-  }
-}
-
-// The CTA takes row `row` of ROWS transforms that share a prime (transform g
-// has limb g mod pm.L for every forward use), so the sub-rows read the same
-// twiddles and the loads hit in L1.
-template <int LOG_N, bool LAZY, class Dst>
-__global__ void __launch_bounds__(Ntt4<LOG_N>::ROW_THREADS)
-    k4_fwd_rows(const uint64_t* buf, Dst dst, PrimeMap pm, int num, CtxDev c) {
-  using S = Ntt4<LOG_N>;
-  using C = typename S::RC;
-  extern __shared__ uint64_t smem[];
-  const int rows = 1 << S::A;
-  const int per_class = num / pm.L;
-  const int groups = (per_class + S::ROWS - 1) / S::ROWS;
-  const int row = blockIdx.x % rows;
-  const int cg = blockIdx.x / rows;
-  const int l = dbg_index(cg / groups, c.L, kDbgLimb), grp = cg % groups;
-  const int sub = threadIdx.x / C::T, tid = threadIdx.x % C::T;
-  const int m = grp * S::ROWS + sub;
-  const bool active = m < per_class;
-  const int g = l + pm.L * (active ? m : per_class - 1);
-  const PrimeDev* P = c.primes + l;
-  const uint64_t q = P->q, two_q = P->two_q;
-  const uint64_t* src = buf + ((size_t)g << LOG_N) + ((size_t)row << S::B);
-  if (active) dst.prefetch(g, l, (row << S::B) | C::fwd_out_idx(tid, 0));
-  uint64_t x[C::E];
-#pragma unroll
-  for (int k = 0; k < C::E; ++k) x[k] = src[C::fwd_in_idx(tid, k)];
-  C::template forward_m<LAZY>(x, tid, RowMap<S::B>{smem, sub},
-                              c.tw_fwd + ((size_t)l << LOG_N), (1 << S::A) + row, q,
-                              two_q);
-  if constexpr (!(LAZY && Dst::kTakesLazy)) finish_fwd<LAZY>(x, q, two_q, P->barrett);
-  // Thread tid holds elements 16 tid .. 16 tid + 15 of its sub-row.  They
-  // go through shared memory (pair slots XOR-swizzled by tid, so neither
-  // side has bank conflicts) and each warp then hands whole sub-rows to the
-  // sink, 32 consecutive pairs per access.
-  static_assert(C::T == 8 && (1 << S::B) == 128 && C::fwd_clo(C::P - 1) == 0,
-                "row epilogue assumes 8 threads x 16 consecutive values per row");
-  __syncthreads();
-  ulonglong2* t2 = reinterpret_cast<ulonglong2*>(smem);
-#pragma unroll
-  for (int p = 0; p < 8; ++p)
-    t2[sub * 64 + tid * 8 + ((p ^ tid) & 7)] = make_ulonglong2(x[2 * p], x[2 * p + 1]);
-  __syncthreads();
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  for (int s2 = warp; s2 < S::ROWS; s2 += S::ROW_THREADS / 32) {
-    const int m2 = grp * S::ROWS + s2;
-    if (m2 >= per_class) break;
-    const auto h = dst.bind(l + pm.L * m2, l, c);
-#pragma unroll
-    for (int half = 0; half < 2; ++half) {
-      const int pp = half * 32 + lane, tq = pp >> 3;
-      const ulonglong2 v = t2[s2 * 64 + tq * 8 + ((pp ^ tq) & 7)];
-      h.pair((row << S::B) + 2 * pp, v.x, v.y);
-    }
   }
 }
 
@@ -914,6 +856,126 @@ __global__ void __launch_bounds__(32 * W, MB)
   }
 }
 
+// Forward row phase: a warp takes four 128-element rows, eight
+// threads with 16 values each per row, so the seven levels are two register
+// passes with one exchange (NttCore<7, 4>) inside the warp.  Its tile holds a row
+// as eight blocks of eight pairs, one pair of padding after each and four between
+// rows: the accesses at 8 k + t, a thread's own eight pairs and whole rows pair by
+// pair all run without bank conflicts at constant offsets.  The results
+// leave through the tile pair by pair, 512 consecutive bytes per warp access.
+// SHARE: the four rows are the same row of four transforms of one prime
+// (blockIdx.y: the class; they read the same twiddles), else four rows of one
+// transform (no idle rows in small batches, four times the twiddles).
+//
+// Bound by the multiply pipe and the latency of its loads; 25 instructions per
+// butterfly where the kernels before it took 33 and more (four two-level passes
+// with three exchanges, or CTA-wide barriers).  n = 2^14, six 45-bit primes: 512
+// polynomials 429 -> 420 us, ModReduce of 256 308 -> 290, the transforms of 200
+// encryptions 278 -> 268.
+struct RowTile64 {
+  static constexpr int kStride = 152;  // words of a row
+  uint64_t* sm;                        // the warp's four rows
+  __device__ __forceinline__ uint64_t* row(int sub) const { return sm + sub * kStride; }
+  template <int k>
+  __device__ __forceinline__ static uint64_t& at(uint64_t* row, int t) {
+    return row[t + 18 * (k >> 1) + 8 * (k & 1)];
+  }
+  __device__ __forceinline__ static ulonglong2* own(uint64_t* row, int t) {
+    return reinterpret_cast<ulonglong2*>(row) + 9 * t;
+  }
+  // Pair 32 h + lane of a row.
+  __device__ __forceinline__ static ulonglong2& lane_pair(uint64_t* row, int lane, int h) {
+    return reinterpret_cast<ulonglong2*>(row)[9 * (lane >> 3) + (lane & 7) + 36 * h];
+  }
+};
+constexpr int kRowWarps = 4;
+constexpr int kRowBytes = kRowWarps * 4 * RowTile64::kStride * 8;
+
+// The rows of one warp: transform and row of each slot.
+template <int LOG_N, bool SHARE>
+struct RowWork {
+  int m0, g0, row0, cls, L, last;
+  __device__ __forceinline__ RowWork(const PrimeMap& pm, int num) {
+    const int item = blockIdx.x * kRowWarps + (threadIdx.x >> 5);
+    L = pm.L;
+    if constexpr (SHARE) {
+      // groups of four fastest: a CTA's warps mostly share the row's twiddles
+      cls = blockIdx.y;
+      last = num / L - 1;
+      const int groups = (last + 4) / 4;
+      row0 = item / groups;
+      m0 = (item - row0 * groups) * 4;
+      g0 = cls + L * m0;
+    } else {
+      constexpr int R4 = 1 << (LOG_N - kNtt4RowBits - 2);
+      g0 = item / R4;
+      row0 = item % R4 * 4;
+      m0 = g0 / L;
+      cls = g0 - m0 * L;
+      last = 0;
+    }
+  }
+  __device__ __forceinline__ int m(int sub) const { return SHARE ? min(m0 + sub, last) : m0; }
+  __device__ __forceinline__ int g(int sub) const { return SHARE ? cls + L * m(sub) : g0; }
+  __device__ __forceinline__ int row(int sub) const { return SHARE ? row0 : row0 + sub; }
+  __device__ __forceinline__ bool active(int sub) const { return !SHARE || m0 + sub <= last; }
+};
+
+template <int LOG_N, bool LAZY, class Dst, bool SHARE>
+__global__ void __launch_bounds__(32 * kRowWarps, 6)
+    k4_fwd_rows(const uint64_t* buf, Dst dst, PrimeMap pm, int num, CtxDev c) {
+  using S = Ntt4<LOG_N>;
+  using C = typename S::RC;
+  __shared__ __align__(16) uint64_t smem[kRowBytes / 8];
+  const RowWork<LOG_N, SHARE> work(pm, num);
+  const int l = dbg_index(work.cls, c.L, kDbgLimb);
+  const int lane = threadIdx.x & 31, sub = lane >> 3, t = lane & 7;
+  const RowTile64 tile{smem + (threadIdx.x >> 5) * 4 * RowTile64::kStride};
+  const PrimeDev* P = c.primes + l;
+  const uint64_t q = P->q, two_q = P->two_q;
+  const Tw* tw = c.tw_fwd + ((size_t)l << LOG_N);
+  const int row = work.row(sub);
+  const uint64_t* src = buf + ((size_t)work.g(sub) << LOG_N) + (row << S::B) + t;
+  if (work.active(sub)) dst.prefetch(work.m(sub), work.g(sub), l, (row << S::B) | (16 * t));
+  uint64_t x[C::E];
+#pragma unroll
+  for (int k = 0; k < C::E; ++k) x[k] = src[8 * k];
+  uint64_t* own_row = tile.row(sub);
+  ulonglong2* own = RowTile64::own(own_row, t);
+  C::template fwd_pass<0, LAZY>(x, t, tw, (1 << S::A) + row, q, two_q);
+  static_for<0, 16>([&](auto k) {
+    RowTile64::at<decltype(k)::value>(own_row, t) = x[decltype(k)::value];
+  });
+  __syncwarp();
+#pragma unroll
+  for (int m = 0; m < 8; ++m) {
+    const ulonglong2 v = own[m];
+    x[2 * m] = v.x;
+    x[2 * m + 1] = v.y;
+  }
+  C::template fwd_pass<1, LAZY>(x, t, tw, (1 << S::A) + row, q, two_q);
+  if constexpr (LAZY && !Dst::kTakesLazy) {
+    const uint32_t mul = P->red_mul, shift = P->red_shift;
+#pragma unroll
+    for (int k = 0; k < C::E; ++k) x[k] = reduce_2q(reduce_1024(x[k], q, mul, shift), q);
+  } else if constexpr (!LAZY) {
+    finish_fwd<LAZY>(x, q, two_q, P->barrett);
+  }
+#pragma unroll
+  for (int m = 0; m < 8; ++m) own[m] = make_ulonglong2(x[2 * m], x[2 * m + 1]);
+  __syncwarp();
+#pragma unroll
+  for (int r = 0; r < 4; ++r) {
+    if (!work.active(r)) break;
+    const auto h = dst.bind(work.m(r), work.g(r), l, c);
+#pragma unroll
+    for (int half = 0; half < 2; ++half) {
+      const ulonglong2 v = RowTile64::lane_pair(tile.row(r), lane, half);
+      h.pair((work.row(r) << S::B) + 2 * (32 * half + lane), v.x, v.y);
+    }
+  }
+}
+
 // Row phases with one warp per row of DPI transforms that share a prime
 // (same twiddles; 4 values per thread per transform, NttCore<7, 2>, four
 // passes exchanged through the warp's own swizzled tiles with warp-level
@@ -950,7 +1012,7 @@ __global__ void __launch_bounds__(32 * W)
   for (int d = 0; d < DPI; ++d) {
     const int mm = min(grp * DPI + d, per_class - 1);
     g[d] = l + pm.L * mm;
-    if (grp * DPI + d < per_class) dst.prefetch(g[d], l, pos0);
+    if (grp * DPI + d < per_class) dst.prefetch(mm, g[d], l, pos0);
     const uint64_t* src = buf + ((size_t)g[d] << LOG_N) + ((size_t)row << S::B);
 #pragma unroll
     for (int e = 0; e < 4; ++e) x[d][e] = src[C::fwd_in_idx(tid, e)];
@@ -974,16 +1036,22 @@ __global__ void __launch_bounds__(32 * W)
   });
 #pragma unroll
   for (int d = 0; d < DPI; ++d) {
-    if constexpr (!(LAZY && Dst::kTakesLazy)) finish_fwd<LAZY>(x[d], q, two_q, P->barrett);
+    if constexpr (LAZY && !Dst::kTakesLazy) {
+#pragma unroll
+      for (int e = 0; e < 4; ++e)
+        x[d][e] = reduce_2q(reduce_1024(x[d][e], q, P->red_mul, P->red_shift), q);
+    } else if constexpr (!LAZY) {
+      finish_fwd<LAZY>(x[d], q, two_q, P->barrett);
+    }
     if (grp * DPI + d < per_class) {
-      const auto h = dst.bind(g[d], l, c);
+      const auto h = dst.bind(grp * DPI + d, g[d], l, c);
       h.pair(pos0, x[d][0], x[d][1]);
       h.pair(pos0 + 2, x[d][2], x[d][3]);
     }
   }
 }
 
-template <int LOG_N, bool WIDE, class Src, int W, int DPI>
+template <int LOG_N, int INV, class Src, int W, int DPI>
 __global__ void __launch_bounds__(32 * W)
     k4_inv_rows_warp(Src src, PrimeMap pm, uint64_t* buf, int num, CtxDev c) {
   using S = Ntt4<LOG_N>;
@@ -1023,7 +1091,7 @@ __global__ void __launch_bounds__(32 * W)
     constexpr int ps = decltype(pp)::value;
 #pragma unroll
     for (int d = 0; d < DPI; ++d)
-      C::template inv_pass<ps, WIDE>(x[d], tid, tw, S::N, 0, row, q, two_q);
+      C::template inv_pass<ps, INV>(x[d], tid, tw, S::N, 0, row, q, two_q);
     if constexpr (ps + 1 < C::P) {
 #pragma unroll
       for (int d = 0; d < DPI; ++d)
@@ -1040,13 +1108,17 @@ __global__ void __launch_bounds__(32 * W)
 #pragma unroll
   for (int d = 0; d < DPI; ++d) {
     if (grp * DPI + d >= per_class) continue;
+    if constexpr (INV == kInvLazy) {  // the last level's sums, for the column phase's [0, 4q)
+#pragma unroll
+      for (int e = 0; e < 2; ++e) x[d][e] = reduce_1024(x[d][e], q, P->red_mul, P->red_shift);
+    }
     uint64_t* dstp = buf + ((size_t)g[d] << LOG_N) + ((size_t)row << S::B);
 #pragma unroll
     for (int e = 0; e < 4; ++e) dstp[C::inv_out_idx(tid, e)] = x[d][e];
   }
 }
 
-template <int LOG_N, bool WIDE, class Src>
+template <int LOG_N, int INV, class Src>
 __global__ void __launch_bounds__(Ntt4<LOG_N>::ROW_THREADS)
     k4_inv_rows(Src src, PrimeMap pm, uint64_t* buf, CtxDev c) {
   using S = Ntt4<LOG_N>;
@@ -1084,14 +1156,19 @@ __global__ void __launch_bounds__(Ntt4<LOG_N>::ROW_THREADS)
     x[2 * p + 1] = v.y;
   }
   __syncthreads();  // the tile is the transform's exchange space next
-  C::template inverse_m<WIDE>(x, tid, RowMap<S::B>{smem, sub}, c.tw_inv + ((size_t)l << LOG_N),
-               S::N, 0, row, q, two_q);
+  C::template inverse_m<INV>(x, tid, RowMap<S::B>{smem, sub}, c.tw_inv + ((size_t)l << LOG_N),
+                             S::N, 0, row, q, two_q);
+  if constexpr (INV == kInvLazy) {  // as in k4_inv_rows_warp
+#pragma unroll
+    for (int k = 0; k < 8; ++k)
+      x[k] = reduce_1024(x[k], q, c.primes[l].red_mul, c.primes[l].red_shift);
+  }
   uint64_t* dst = buf + ((size_t)g << LOG_N) + ((size_t)row << S::B);
 #pragma unroll
   for (int k = 0; k < C::E; ++k) dst[C::inv_out_idx(tid, k)] = x[k];
 }
 
-template <int LOG_N, bool WIDE, class Dst>
+template <int LOG_N, int INV, class Dst>
 __global__ void __launch_bounds__(Ntt4<LOG_N>::COL_THREADS)
     k4_inv_cols(const uint64_t* buf, Dst dst, PrimeMap pm, CtxDev c) {
   using S = Ntt4<LOG_N>;
@@ -1106,30 +1183,42 @@ __global__ void __launch_bounds__(Ntt4<LOG_N>::COL_THREADS)
   uint64_t x[C::E];
 #pragma unroll
   for (int k = 0; k < C::E; ++k) x[k] = src[(C::inv_in_idx(t, k) << S::B) | col];
-  C::template inverse_m<WIDE>(x, t, typename C::ColMap{smem, S::COLS, j},
+  C::template inverse_m<INV>(x, t, typename C::ColMap{smem, S::COLS, j},
                c.tw_inv + ((size_t)l << LOG_N), S::N, S::B, 0, q, two_q);
   const auto h = dst.bind(g, l, c);
 #pragma unroll
   for (int k = 0; k < C::E; ++k) h((C::inv_out_idx(t, k) << S::B) | col, x[k]);
 }
 
-// Forward row phase grid: (prime class, group of ROWS transforms, row).
-// Every forward caller passes PrimeMap{0, 1, L} with num a multiple of L.
+// Row-phase choice (measured on a GB300): k4_fwd_rows for the plain, ModReduce and
+// encryption sinks; the warp-per-row kernels, three transforms of one prime per
+// warp, for the key switch's last rows (28.5 against 33 us per 16 ciphertexts at
+// n = 2^14, six limbs) and for the plain and component sources of the inverse; the
+// CTA-per-row kernel for the tensor source, whose loads want 32 consecutive pairs
+// per warp access.
+constexpr int kRowsWarpW = 4, kRowsWarpDpi = 3;
+
+// Row launch: four transforms of one prime share a row where the classes fill at
+// least four fifths of the groups.
+inline bool share_rows(int num, int L) {
+  const int per = num / L;
+  return num % L == 0 && per >= 3 && (per + 3) / 4 * 4 * 8 <= per * 10;
+}
 template <int LOG_N>
-int row_blocks(int num, PrimeMap pm) {
-  using S = Ntt4<LOG_N>;
-  const int per_class = num / pm.L;
-  const int groups = (per_class + S::ROWS - 1) / S::ROWS;
-  return pm.L * groups * (1 << S::A);
+dim3 row_grid(int num, int L, bool share) {
+  constexpr int R = 1 << (LOG_N - kNtt4RowBits);
+  return share ? dim3(R * ((num / L + 3) / 4) / kRowWarps, L) : dim3(num * (R / 4) / kRowWarps);
 }
 
-// Row-phase choice (measured on a GB300, n = 2^14 and 2^15): the warp-per-row
-// kernels, three transforms of one prime per warp, are 2-3 % faster for the
-// plain sink and for the plain and component sources; the CTA-per-row
-// kernels stay faster for the fused sinks (encryption, ModReduce), whose
-// loads want 32 consecutive pairs per warp access, and for the tensor
-// source.
-constexpr int kRowsWarpW = 4, kRowsWarpDpi = 3;
+template <int LOG_N, class Dst>
+void fwd_rows4(const CtxDev& c, const uint64_t* buf, const Dst& dst, PrimeMap pm, int num,
+               bool lazy, cudaStream_t s) {
+  const bool share = share_rows(num, pm.L);
+  auto k2 = share ? (lazy ? k4_fwd_rows<LOG_N, true, Dst, true> : k4_fwd_rows<LOG_N, false, Dst, true>)
+                  : (lazy ? k4_fwd_rows<LOG_N, true, Dst, false>
+                          : k4_fwd_rows<LOG_N, false, Dst, false>);
+  k2<<<row_grid<LOG_N>(num, pm.L, share), 32 * kRowWarps, 0, s>>>(buf, dst, pm, num, c);
+}
 
 template <int LOG_N, class Src, class Dst>
 void fwd4(const CtxDev& c, const Src& src, const Dst& dst, PrimeMap pm,
@@ -1149,43 +1238,40 @@ void fwd4(const CtxDev& c, const Src& src, const Dst& dst, PrimeMap pm,
     cols(std::true_type{});
   else
     cols(std::false_type{});
-  if constexpr (std::is_same_v<Dst, FwdDstPlain<LOG_N>>) {
-    constexpr int W = kRowsWarpW, DPI = kRowsWarpDpi;
-    const int groups = (num / pm.L + DPI - 1) / DPI;
-    const int blocks = pm.L * groups * (1 << S::A) / W;
-    auto k2 = c.small_q ? k4_fwd_rows_warp<LOG_N, true, Dst, W, DPI>
-                        : k4_fwd_rows_warp<LOG_N, false, Dst, W, DPI>;
-    set_smem4(k2, W * DPI * (1 << S::B) * 8);
-    k2<<<blocks, 32 * W, W * DPI * (1 << S::B) * 8, s>>>(buf, dst, pm, num, c);
-  } else {
-    auto k2 = c.small_q ? k4_fwd_rows<LOG_N, true, Dst> : k4_fwd_rows<LOG_N, false, Dst>;
-    set_smem4(k2, S::ROW_SMEM);
-    k2<<<row_blocks<LOG_N>(num, pm), S::ROW_THREADS, S::ROW_SMEM, s>>>(buf, dst, pm,
-                                                                      num, c);
-  }
+  fwd_rows4<LOG_N>(c, buf, dst, pm, num, c.small_q != 0, s);
 }
 
-template <int LOG_N, class Src, class Dst>
-void inv4(const CtxDev& c, const Src& src, const Dst& dst, PrimeMap pm,
-          uint64_t* buf, int num, cudaStream_t s) {
+template <int LOG_N, int INV, class Src, class Dst>
+void inv4_mode(const CtxDev& c, const Src& src, const Dst& dst, PrimeMap pm,
+               uint64_t* buf, int num, cudaStream_t s) {
   using S = Ntt4<LOG_N>;
-  auto k2 = c.small_q ? k4_inv_cols<LOG_N, true, Dst> : k4_inv_cols<LOG_N, false, Dst>;
+  auto k2 = k4_inv_cols<LOG_N, INV, Dst>;
   set_smem4(k2, S::COL_SMEM);
   constexpr bool warp_rows = std::is_same_v<Src, InvSrcPlain<LOG_N>> ||
                              std::is_same_v<Src, InvSrcComponent<LOG_N>>;
   if (warp_rows && num % pm.L == 0) {
     constexpr int W = kRowsWarpW, DPI = kRowsWarpDpi;
     const int groups = pm.L * ((num / pm.L + DPI - 1) / DPI);
-    auto k1 = c.small_q ? k4_inv_rows_warp<LOG_N, true, Src, W, DPI>
-                        : k4_inv_rows_warp<LOG_N, false, Src, W, DPI>;
+    auto k1 = k4_inv_rows_warp<LOG_N, INV, Src, W, DPI>;
     set_smem4(k1, W * DPI * (1 << S::B) * 8);
     k1<<<groups * (1 << S::A) / W, 32 * W, W * DPI * (1 << S::B) * 8, s>>>(src, pm, buf, num, c);
   } else {
-    auto k1 = c.small_q ? k4_inv_rows<LOG_N, true, Src> : k4_inv_rows<LOG_N, false, Src>;
+    auto k1 = k4_inv_rows<LOG_N, INV, Src>;
     set_smem4(k1, S::ROW_SMEM);
     k1<<<num * S::ROW_TILES, S::ROW_THREADS, S::ROW_SMEM, s>>>(src, pm, buf, c);
   }
   k2<<<num * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s>>>(buf, dst, pm, c);
+}
+
+template <int LOG_N, class Src, class Dst>
+void inv4(const CtxDev& c, const Src& src, const Dst& dst, PrimeMap pm,
+          uint64_t* buf, int num, cudaStream_t s) {
+  if (c.lazy_inv)
+    inv4_mode<LOG_N, kInvLazy>(c, src, dst, pm, buf, num, s);
+  else if (c.small_q)
+    inv4_mode<LOG_N, kInvWide>(c, src, dst, pm, buf, num, s);
+  else
+    inv4_mode<LOG_N, kInvExact>(c, src, dst, pm, buf, num, s);
 }
 
 #define SHG_DISPATCH4(log_n, F) \
