@@ -1232,7 +1232,7 @@ BFV_METRIC = "RNS BFV ct*ct/sec (RnsBfvCiphertext::Mul, bit-exact)"
 BFV_UNIT = "bfv-mul/s"
 P45_AUX = [35184368320513, 35184368025601, 35184367828993, 35184367337473, 35184366911489,
            35184366551041, 35184366223361]
-BFV_SCOPES = ("ntt_inv", "ntt_fwd", "switch_basis", "tensor", "lin2")
+BFV_SCOPES = ("ntt_inv", "ntt_fwd", "switch_basis", "tensor", "ntt_fwd_combine")
 
 
 def bfv_config(count):
@@ -1245,8 +1245,9 @@ def bfv_config(count):
 def bfv_scope_model(name, n, Lm, K, pairs):
     """Algorithmic DRAM bytes of one step of a scope (limb = n * 8 bytes)."""
     limb = n * 8
-    per = {"ntt_inv": 2 * (4 * Lm + 3 * K), "ntt_fwd": 2 * (2 * K + 2 * Lm + 2 * K + 3 * Lm),
-           "switch_basis": 9 * (Lm + K), "tensor": 7 * Lm + 7 * K, "lin2": 9 * Lm}[name]
+    per = {"ntt_inv": 2 * (4 * Lm + 3 * K), "ntt_fwd": 2 * (4 * K + 2 * Lm),
+           "switch_basis": 9 * (Lm + K), "tensor": 7 * Lm + 7 * K,
+           "ntt_fwd_combine": 9 * Lm}[name]
     return per * limb * pairs
 
 
@@ -1417,7 +1418,8 @@ def run_bfv(args, world, rank, local, dist):
     step_total = sum(v[0] for v in prof.values())
     kernels = {}
     limb_bfly = n // 2 * LOG_N
-    bfly_limbs = {"ntt_inv": 4 * L + 3 * K, "ntt_fwd": 4 * K + 5 * L}
+    bfly_limbs = {"ntt_inv": 4 * L + 3 * K, "ntt_fwd": 4 * K + 2 * L,
+                  "ntt_fwd_combine": 3 * L}
     for name, (ms, cnt) in prof.items():
         nbytes = bfv_scope_model(name, n, L, K, B)
         kernels[name] = {"share_of_step": ms / step_total, "launches": cnt,

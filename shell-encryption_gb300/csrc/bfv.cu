@@ -47,8 +47,10 @@ __device__ __forceinline__ uint64_t round_sum(const uint64_t (&v)[MAXS], const u
 // accumulation per destination value (the host sets `fast` only when every
 // sum_i v_i w_ij + u z_j stays below p_j 2^64), unbalanced.  Each thread
 // converts coefficients k and k + n/2 of one member, so every table value
-// read from shared memory serves two independent carry chains.
-template <int NS>
+// read from shared memory serves two independent carry chains.  NARROW (primes
+// below 2^45): the products' high words vanish and u is a few bits, so each
+// multiply-accumulate saves a multiply and u's four.
+template <int NS, bool NARROW>
 __global__ void __launch_bounds__(kConvThreads, NS >= 8 ? 2 : 3)
     k_switch_basis_ns(const BasisConv* __restrict__ bcp, const PrimeDev* __restrict__ primes,
                       const uint64_t* __restrict__ in, size_t in_stride,
@@ -115,13 +117,26 @@ __global__ void __launch_bounds__(kConvThreads, NS >= 8 ? 2 : 3)
 #pragma unroll
       for (int i = 0; i < NS; ++i) {
         const uint64_t wi = w[i];
-        mac128(lo0, hi0, v0[i], wi);
-        mac128(lo1, hi1, v1[i], wi);
+        if constexpr (NARROW) {
+          mac128_narrow(lo0, hi0, v0[i], wi);
+          mac128_narrow(lo1, hi1, v1[i], wi);
+        } else {
+          mac128(lo0, hi0, v0[i], wi);
+          mac128(lo1, hi1, v1[i], wi);
+        }
       }
       if (with_u) {
         const uint64_t z = d_z[j];
-        mac128(lo0, hi0, u0, z);
-        mac128(lo1, hi1, u1, z);
+        if constexpr (NARROW) {  // u <= NS, z < 2^45: no high word
+          const uint64_t t0 = u0 * z, t1 = u1 * z;
+          lo0 += t0;
+          hi0 += lo0 < t0;
+          lo1 += t1;
+          hi1 += lo1 < t1;
+        } else {
+          mac128(lo0, hi0, u0, z);
+          mac128(lo1, hi1, u1, z);
+        }
       }
       const uint64_t q = d_q[j], qinv = d_qinv[j];
       o[(size_t)j << log_n] = redc128(lo0, hi0, q, qinv);
@@ -220,8 +235,9 @@ void launch_switch_basis(const PrimeDev* primes, ConvRef conv, int ns, int nd,
     const int grid = grid_for(total / 2, kConvThreads);
 #define SHG_SWITCH_NS(NS)                                                                   \
   case NS:                                                                                  \
-    k_switch_basis_ns<NS><<<grid, kConvThreads, smem, s>>>(bc, primes, in, in_stride, out, \
-                                                           out_stride, total / 2, log_n);   \
+    (conv.narrow ? k_switch_basis_ns<NS, true> : k_switch_basis_ns<NS, false>)              \
+        <<<grid, kConvThreads, smem, s>>>(bc, primes, in, in_stride, out, out_stride,       \
+                                          total / 2, log_n);                                \
     return;
     switch (ns) {
       SHG_SWITCH_NS(1)

@@ -2454,7 +2454,7 @@ static int check_aux(shg_context* ctx, int count, int num_limbs) {
 
 static shg::ConvRef conv(const shg_context* ctx, int kind, int level, int balanced = 0) {
   const int slot = conv_slot(ctx, kind, level, balanced);
-  return shg::ConvRef{ctx->d_conv + slot, ctx->conv_fast[slot]};
+  return shg::ConvRef{ctx->d_conv + slot, ctx->conv_fast[slot], ctx->narrow_q};
 }
 
 int shg_poly_switch_rns_basis(shg_context* ctx, uint64_t* out, const uint64_t* in,
@@ -2686,12 +2686,21 @@ static void bfv_scale_reduce(shg_context* ctx, uint64_t* out, const uint64_t* t_
   shg::launch_ntt_inv(ctx->aux_dev(), t_aux, t_aux, count * K, K, 0, s);
   shg::launch_switch_basis(ctx->d_primes, conv(ctx, CONV_SWITCH_DOWN_T, Lm - 1), K, Lm, t_aux,
                            (size_t)K * n, D, (size_t)Lm * n, count, ctx->log_n, s);
-  shg::launch_ntt_fwd(ctx->dev(), D, D, count * Lm, Lm, s);
+  // out = (t t_main - D) P^-1, in the last row phase of D's transform where it
+  // runs on the four-step kernels
   std::vector<uint64_t> c(Lm), d(Lm);
+  shg::ScalarPack sc{};
   for (int i = 0; i < Lm; ++i) {
+    const uint64_t q = ctx->hp[i].q;
     d[i] = p_inv_mod(ctx, i);
-    c[i] = mulmod(ctx->t % ctx->hp[i].q, d[i], ctx->hp[i].q);
+    c[i] = mulmod(ctx->t % q, d[i], q);
+    sc.v[4 * i] = c[i];
+    sc.v[4 * i + 1] = shoup_of(c[i], q);
+    sc.v[4 * i + 2] = q - d[i];
+    sc.v[4 * i + 3] = shoup_of(q - d[i], q);
   }
+  if (shg::launch4_ntt_fwd_combine(ctx->dev(), out, D, t_main, sc, count, Lm, s)) return;
+  shg::launch_ntt_fwd(ctx->dev(), D, D, count * Lm, Lm, s);
   combine(ctx, out, t_main, D, c.data(), d.data(), 1, count, Lm, s);
 }
 
@@ -2707,31 +2716,49 @@ int shg_bfv_mul(shg_context* ctx, uint64_t* out, const uint64_t* a, const uint64
   // per ciphertext: X [4][Lm] (a, b coefficient forms; later the deltas),
   // b_aux [2][K], a_aux [2][K], a_main [2][Lm], t_main [3][Lm], t_aux [3][K]
   const size_t per_ct = (9 * pm + 7 * pa) * sizeof(uint64_t);
-  const size_t want = ctx->chunk_cts > 0 ? (size_t)ctx->chunk_cts
-                                         : std::max<size_t>(1, ((size_t)1 << 30) / per_ct);
-  const int C = (int)std::min<size_t>((size_t)count, want);
+  // Chunks of 256 MB on the key-switch lanes, two of them from eight pairs on, or
+  // of one GiB where there is one lane: 96 pairs at n = 2^14, 6 + 7 primes take
+  // 2326 us so, 2633 on one stream (before the combine below was fused: 2448 us
+  // with 256 MB on two lanes, 2467 with 512 MB, 2637 with 128 MB, 3243 with 64 MB).
   std::lock_guard<std::mutex> lock(ctx->mu);
-  if ((st = ctx->ensure_ws((size_t)C * per_ct))) return st;
-  uint64_t* X = ctx->ws;
-  uint64_t* b_aux = X + (size_t)C * 4 * pm;
-  uint64_t* a_aux = b_aux + (size_t)C * 2 * pa;
-  uint64_t* a_main = a_aux + (size_t)C * 2 * pa;
-  uint64_t* t_main = a_main + (size_t)C * 2 * pm;
-  uint64_t* t_aux = t_main + (size_t)C * 3 * pm;
-  for (int c0 = 0; c0 < count; c0 += C) {
-    const int cc = std::min(C, count - c0);
+  KsLanes lanes{ctx, s};
+  if ((st = lanes.open(count >= 8 ? 2 : 1))) return st;
+  const size_t most =
+      std::max<size_t>(1, ((size_t)(lanes.n > 1 ? 256 : 1024) << 20) / per_ct);
+  const size_t want = ctx->chunk_cts > 0 ? (size_t)ctx->chunk_cts
+                      : lanes.n > 1      ? std::min<size_t>(most, (count + 1) / 2)
+                                         : most;
+  const int C = (int)std::min<size_t>((size_t)count, want);
+  const int nchunks = (count + C - 1) / C;
+  // Never less than one lane's chunks of this batch: a smaller batch, or one on a
+  // single lane, then fits the scratch that a larger one left (a capture cannot grow it).
+  const size_t alone = ctx->chunk_cts > 0 ? (size_t)ctx->chunk_cts
+                                          : std::max<size_t>(1, ((size_t)1 << 30) / per_ct);
+  const size_t scratch_cts = std::max((size_t)lanes.n * C, std::min<size_t>(count, alone));
+  if ((st = ctx->ensure_ws(scratch_cts * per_ct))) return st;
+  if ((st = lanes.fork())) return st;
+  for (int i = 0; i < nchunks; ++i) {
+    const int c0 = i * C, cc = std::min(C, count - c0), lane = i % lanes.n;
+    cudaStream_t ls = lanes.stream(lane);
+    uint64_t* X = ctx->ws + lane * C * per_ct / sizeof(uint64_t);
+    uint64_t* b_aux = X + (size_t)C * 4 * pm;
+    uint64_t* a_aux = b_aux + (size_t)C * 2 * pa;
+    uint64_t* a_main = a_aux + (size_t)C * 2 * pa;
+    uint64_t* t_main = a_main + (size_t)C * 2 * pm;
+    uint64_t* t_aux = t_main + (size_t)C * 3 * pm;
     const uint64_t* ac = a + (size_t)c0 * 2 * pm;
     const uint64_t* bc = b + (size_t)c0 * 2 * pm;
     // Q/t * b_j (mod P): b -> coefficient form -> SwitchRnsBasis -> NTT
-    bfv_switch_up(ctx, bc, X, b_aux, cc * 2, Lm, s);
+    bfv_switch_up(ctx, bc, X, b_aux, cc * 2, Lm, ls);
     // P/t * a_i (mod P) and (mod Q)
-    bfv_scale_up(ctx, ac, X, a_aux, a_main, cc * 2, Lm, s);
+    bfv_scale_up(ctx, ac, X, a_aux, a_main, cc * 2, Lm, ls);
     // the tensor product mod Q and mod P
-    shg::launch_tensor(ctx->dev(), t_main, a_main, bc, cc, Lm, s);
-    shg::launch_tensor(ctx->aux_dev(), t_aux, a_aux, b_aux, cc, K, s);
+    shg::launch_tensor(ctx->dev(), t_main, a_main, bc, cc, Lm, ls);
+    shg::launch_tensor(ctx->aux_dev(), t_aux, a_aux, b_aux, cc, K, ls);
     // Q/t * tensor (mod Q)
-    bfv_scale_reduce(ctx, out + (size_t)c0 * 3 * pm, t_main, t_aux, X, cc * 3, Lm, s);
+    bfv_scale_reduce(ctx, out + (size_t)c0 * 3 * pm, t_main, t_aux, X, cc * 3, Lm, ls);
   }
+  if ((st = lanes.join())) return st;
   return launch_status("bfv_mul");
 }
 

@@ -428,24 +428,23 @@ __global__ void k_substitute(uint64_t* out, const uint64_t* in, int power,
   }
 }
 
-__global__ void k_tensor(uint64_t* out, const uint64_t* a, const uint64_t* b,
-                         size_t total /* count*L*n */, int log_n, int L,
-                         CtxDev c) {
+// Two adjacent coefficients of ciphertexts blockIdx.y, + gridDim.y, ... per thread.
+__global__ void k_tensor(uint64_t* out, const uint64_t* a, const uint64_t* b, int count,
+                         int log_n, int L, CtxDev c) {
   const size_t Ln = (size_t)L << log_n;
-  const size_t stride = (size_t)gridDim.x * blockDim.x;
-  for (size_t e = (size_t)blockIdx.x * blockDim.x + threadIdx.x; e < total;
-       e += stride) {
-    const size_t ct = e / Ln, r = e % Ln;
-    const int l = (int)(r >> log_n);
-    const PrimeDev* P = c.primes + l;
-    const uint64_t q = P->q, qinv = P->inv_modulus;
-    const uint64_t a0 = a[ct * 2 * Ln + r], a1 = a[ct * 2 * Ln + Ln + r];
-    const uint64_t b0 = b[ct * 2 * Ln + r], b1 = b[ct * 2 * Ln + Ln + r];
-    uint64_t c0, c1, c2;
-    tensor3(a0, a1, b0, b1, q, qinv, c0, c1, c2);
-    out[ct * 3 * Ln + r] = c0;
-    out[ct * 3 * Ln + Ln + r] = c1;
-    out[ct * 3 * Ln + 2 * Ln + r] = c2;
+  const size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
+  if (r >= Ln) return;
+  const PrimeDev* P = c.primes + (r >> log_n);
+  const uint64_t q = P->q, qinv = P->inv_modulus;
+  auto at = [](const uint64_t* p) { return *reinterpret_cast<const ulonglong2*>(p); };
+  for (size_t ct = blockIdx.y; ct < (size_t)count; ct += gridDim.y) {
+    const uint64_t *pa = a + ct * 2 * Ln + r, *pb = b + ct * 2 * Ln + r;
+    ulonglong2 c0, c1, c2;
+    tensor3_pair(at(pa), at(pa + Ln), at(pb), at(pb + Ln), q, qinv, c0, c1, c2);
+    uint64_t* o = out + ct * 3 * Ln + r;
+    *reinterpret_cast<ulonglong2*>(o) = c0;
+    *reinterpret_cast<ulonglong2*>(o + Ln) = c1;
+    *reinterpret_cast<ulonglong2*>(o + 2 * Ln) = c2;
   }
 }
 
@@ -1132,8 +1131,8 @@ void launch_tensor(const CtxDev& c, uint64_t* out, const uint64_t* a,
   const size_t total = (size_t)count * L * c.n;
   if (total == 0) return;
   LaunchScope scope_("tensor", s);
-  k_tensor<<<grid_for(total, 256), 256, 0, s>>>(out, a, b, total, c.log_n, L,
-                                                c);
+  const dim3 grid((unsigned)(((size_t)L * c.n / 2 + 255) / 256), std::min(count, 65535));
+  k_tensor<<<grid, 256, 0, s>>>(out, a, b, count, c.log_n, L, c);
 }
 
 void launch_tensor_intt(const CtxDev& c, uint64_t* out01, uint64_t* X,

@@ -368,6 +368,7 @@ struct BasisConv {
 struct ConvRef {
   const BasisConv* bc;
   int fast;
+  int narrow;  // every prime of the context below 2^45 (mac128_narrow)
 };
 
 void launch_switch_basis(const PrimeDev* primes, ConvRef conv, int ns, int nd,
@@ -471,6 +472,11 @@ void launch4_digit_ntt(const CtxDev& c, uint64_t* D, const uint64_t* X,
 void launch4_modreduce_lift(const CtxDev& c, uint64_t* out, const uint64_t* Y,
                             const uint64_t* in, const ScalarPack& sc, int count,
                             int L, cudaStream_t s);
+
+// out = in * c1 + NTT(x) * c2 per limb (sc as in launch_modreduce_ntt), all
+// [count][L][n], x used up; false below the four-step plain-NTT range.
+bool launch4_ntt_fwd_combine(const CtxDev& c, uint64_t* out, uint64_t* x, const uint64_t* in,
+                             const ScalarPack& sc, int count, int L, cudaStream_t s);
 
 // Fused four-step encryption tail: NTT of the lifted error err [count][n]
 // with the combine of launch_bgv_enc_combine as its sink; buf [count][L][n].

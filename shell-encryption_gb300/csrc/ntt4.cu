@@ -153,7 +153,7 @@ struct FwdDstPlain {
 };
 
 // ModReduceLsb combine: out_i = in_i * c1 + delta_i * c2
-// (rns/rns_polynomial.cc:314-323).
+// (rns/rns_polynomial.cc:314-323); `in` has L limbs per polynomial.
 template <int LOG_N>
 struct FwdDstModCombine {
   // Shoup products take any 64-bit x, so lazily reduced values need no
@@ -1468,6 +1468,19 @@ void launch4_modreduce_lift(const CtxDev& c, uint64_t* out, const uint64_t* Y,
            PrimeMap{0, 1, L - 1}, out, count * (L - 1), s)
   SHG_DISPATCH4(c.log_n, F)
 #undef F
+}
+
+bool launch4_ntt_fwd_combine(const CtxDev& c, uint64_t* out, uint64_t* x, const uint64_t* in,
+                             const ScalarPack& sc, int count, int L, cudaStream_t s) {
+  if (c.log_n < 12 || (c.log_n < c.ntt4_plain_min && c.log_n <= 14)) return false;
+  LaunchScope scope_("ntt_fwd_combine", s);
+  g_launch_count++;  // second phase kernel
+#define F(LN)                                                                       \
+  fwd4<LN>(c, FwdSrcPlain<LN>{x}, FwdDstModCombine<LN>{out, in, L, sc},              \
+           PrimeMap{0, 1, L}, x, count * L, s)
+  SHG_DISPATCH4(c.log_n, F)
+#undef F
+  return true;
 }
 
 void launch4_bgv_encrypt(const CtxDev& c, uint64_t* out, const int32_t* err,
