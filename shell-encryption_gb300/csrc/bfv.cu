@@ -56,6 +56,7 @@ __global__ void __launch_bounds__(kConvThreads, NS >= 8 ? 2 : 3)
                       const uint64_t* __restrict__ in, size_t in_stride,
                       uint64_t* __restrict__ out, size_t out_stride, size_t total_half,
                       int log_n) {
+  after_previous();
   extern __shared__ uint64_t tab[];
   const BasisConv& bc = *bcp;
   const int nd = bc.nd;
@@ -225,7 +226,7 @@ __global__ void k_lin2(uint64_t* out, const uint64_t* a, const uint64_t* b, Scal
 
 void launch_switch_basis(const PrimeDev* primes, ConvRef conv, int ns, int nd,
                          const uint64_t* in, size_t in_stride, uint64_t* out,
-                         size_t out_stride, int count, int log_n, cudaStream_t s) {
+                         size_t out_stride, int count, int log_n, cudaStream_t s, bool follows) {
   const size_t total = (size_t)count << log_n;
   if (total == 0 || nd == 0) return;
   LaunchScope scope_("switch_basis", s);
@@ -235,9 +236,9 @@ void launch_switch_basis(const PrimeDev* primes, ConvRef conv, int ns, int nd,
     const int grid = grid_for(total / 2, kConvThreads);
 #define SHG_SWITCH_NS(NS)                                                                   \
   case NS:                                                                                  \
-    (conv.narrow ? k_switch_basis_ns<NS, true> : k_switch_basis_ns<NS, false>)              \
-        <<<grid, kConvThreads, smem, s>>>(bc, primes, in, in_stride, out, out_stride,       \
-                                          total / 2, log_n);                                \
+    launch_next(follows, conv.narrow ? k_switch_basis_ns<NS, true> : k_switch_basis_ns<NS, false>, \
+                grid, kConvThreads, smem, s, bc, primes, in, in_stride, out, out_stride,    \
+                total / 2, log_n);                                                          \
     return;
     switch (ns) {
       SHG_SWITCH_NS(1)

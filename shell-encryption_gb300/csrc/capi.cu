@@ -1286,8 +1286,8 @@ int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
                             CtMap::identity(), cc, L, lanes.stream(lane));
     shg::KeyTable kt;
     if (keys) kt = shg::KeyTable{table.kb + c0, table.ka + c0, 0, count - c0};
-    shg::launch_keyswitch(dv, D, X, key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
-                          key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src,
+    shg::launch_keyswitch(dv.next(), D, X, key->d_digits, k, key->digit_flags, key->chunk,
+                          key->chunk_lazy, key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src,
                           (size_t)a.ncomp * Ln, CtMap::identity(), a.base1_zero,
                           a.subst_power, cc, L, lanes.stream(lane), kt, ks32);
   }
@@ -1387,8 +1387,9 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
     uint64_t* o = out + (size_t)c0 * 2 * Ln;
     shg::KeyTable kc;
     if (keys) kc = shg::KeyTable{kt.kb + c0, kt.ka + c0, 0, count - c0};
-    shg::launch_keyswitch(dv, D0 + lane * C * d_per_ct / 8, X + (size_t)c0 * Ln,
-                          key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
+    // the first on a side lane follows an event wait
+    shg::launch_keyswitch(lanes == 1 ? dv.next() : dv, D0 + lane * C * d_per_ct / 8,
+                          X + (size_t)c0 * Ln, key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
                           key->kb, key->ka, o, o, 2 * Ln, CtMap::identity(), 0, 0, cc, L, ls,
                           kc, ks32);
   }
@@ -1855,12 +1856,12 @@ int run_expand(shg_context* ctx, const shg_key* const* keys, int levels, uint64_
   // on the stream so the whole expansion can be captured in a graph.
   shg::launch_monomials(ctx->dev(), mono, levels, ctx->hp[0].q - ctx->hp[0].r_mod_q, s);
   shg::launch_ntt_fwd(ctx->dev(), mono, mono, levels, 1, s);
-  const CtxDev dv = ctx->dev();
   // Queries are independent: each lane takes its share of them through all
   // levels with its own X, D and KS, so one lane's memory-bound level update
   // runs beside another's digit transforms (24 queries of 10 levels at
   // n = 2^12: 12.8 -> 11.3 ms).
   KsLanes lanes{ctx, s, plan.lanes};
+  const CtxDev dv = ctx->dev();
   int st = lanes.fork();
   if (st) return st;
   const int share = (count + plan.lanes - 1) / plan.lanes;
@@ -1885,11 +1886,11 @@ int run_expand(shg_context* ctx, const shg_key* const* keys, int levels, uint64_
         if (tables)
           kt = shg::KeyTable{tables[j].kb + q0, tables[j].ka + q0, j,
                              tables[j].entries ? tables[j].entries - q0 : 0};
-        if (shg::launch_ks_expand(dv, blk, D, X, key->d_digits, key->k, key->digit_flags,
+        if (shg::launch_ks_expand(dv.next(), blk, D, X, key->d_digits, key->k, key->digit_flags,
                                   key->chunk, key->chunk_lazy, key->kb, key->ka,
                                   mono + (size_t)j * n, map, j, power, mc, ls, kt))
           continue;
-        shg::launch_keyswitch(dv, D, X, key->d_digits, key->k, key->digit_flags, key->chunk,
+        shg::launch_keyswitch(dv.next(), D, X, key->d_digits, key->k, key->digit_flags, key->chunk,
                               key->chunk_lazy, key->kb, key->ka, KS, blk, 2 * (size_t)n, map, 1,
                               power, mc, 1, ls, kt);
         shg::launch_expand_combine(dv, blk, KS, mono + (size_t)j * n, map, 1 << j, mc, ls);
@@ -2658,11 +2659,11 @@ static void bfv_scale_up(shg_context* ctx, const uint64_t* x, uint64_t* X, uint6
   const int K = ctx->K, l = Lm - 1;
   shg::launch_ntt_inv(ctx->dev(), x, X, count * Lm, Lm, 0, s);
   shg::launch_switch_basis(ctx->d_primes, conv(ctx, CONV_SCALE_UP, l), Lm, K, X,
-                           (size_t)Lm * n, x_aux, (size_t)K * n, count, ctx->log_n, s);
+                           (size_t)Lm * n, x_aux, (size_t)K * n, count, ctx->log_n, s, true);
   shg::launch_switch_basis(ctx->d_primes, conv(ctx, CONV_SWITCH_DOWN, l), K, Lm, x_aux,
-                           (size_t)K * n, x_main, (size_t)Lm * n, count, ctx->log_n, s);
-  shg::launch_ntt_fwd(ctx->dev(), x_main, x_main, count * Lm, Lm, s);
-  shg::launch_ntt_fwd(ctx->aux_dev(), x_aux, x_aux, count * K, K, s);
+                           (size_t)K * n, x_main, (size_t)Lm * n, count, ctx->log_n, s, true);
+  shg::launch_ntt_fwd(ctx->dev().next(), x_main, x_main, count * Lm, Lm, s);
+  shg::launch_ntt_fwd(ctx->aux_dev().next(), x_aux, x_aux, count * K, K, s);
 }
 
 // NTT-form x [count][Lm][n] -> its SwitchRnsBasis to the auxiliary primes in
@@ -2673,8 +2674,8 @@ static void bfv_switch_up(shg_context* ctx, const uint64_t* x, uint64_t* X, uint
   const int K = ctx->K;
   shg::launch_ntt_inv(ctx->dev(), x, X, count * Lm, Lm, 0, s);
   shg::launch_switch_basis(ctx->d_primes, conv(ctx, CONV_SWITCH_UP, Lm - 1), Lm, K, X,
-                           (size_t)Lm * n, x_aux, (size_t)K * n, count, ctx->log_n, s);
-  shg::launch_ntt_fwd(ctx->aux_dev(), x_aux, x_aux, count * K, K, s);
+                           (size_t)Lm * n, x_aux, (size_t)K * n, count, ctx->log_n, s, true);
+  shg::launch_ntt_fwd(ctx->aux_dev().next(), x_aux, x_aux, count * K, K, s);
 }
 
 // ScaleAndReduceRnsBasisInPlace with the context's t of (t_main, t_aux) [count]
@@ -2683,9 +2684,9 @@ static void bfv_scale_reduce(shg_context* ctx, uint64_t* out, const uint64_t* t_
                              uint64_t* t_aux, uint64_t* D, int count, int Lm, cudaStream_t s) {
   const size_t n = ctx->n;
   const int K = ctx->K;
-  shg::launch_ntt_inv(ctx->aux_dev(), t_aux, t_aux, count * K, K, 0, s);
+  shg::launch_ntt_inv(ctx->aux_dev().next(), t_aux, t_aux, count * K, K, 0, s);
   shg::launch_switch_basis(ctx->d_primes, conv(ctx, CONV_SWITCH_DOWN_T, Lm - 1), K, Lm, t_aux,
-                           (size_t)K * n, D, (size_t)Lm * n, count, ctx->log_n, s);
+                           (size_t)K * n, D, (size_t)Lm * n, count, ctx->log_n, s, true);
   // out = (t t_main - D) P^-1, in the last row phase of D's transform where it
   // runs on the four-step kernels
   std::vector<uint64_t> c(Lm), d(Lm);
@@ -2699,7 +2700,7 @@ static void bfv_scale_reduce(shg_context* ctx, uint64_t* out, const uint64_t* t_
     sc.v[4 * i + 2] = q - d[i];
     sc.v[4 * i + 3] = shoup_of(q - d[i], q);
   }
-  if (shg::launch4_ntt_fwd_combine(ctx->dev(), out, D, t_main, sc, count, Lm, s)) return;
+  if (shg::launch4_ntt_fwd_combine(ctx->dev().next(), out, D, t_main, sc, count, Lm, s)) return;
   shg::launch_ntt_fwd(ctx->dev(), D, D, count * Lm, Lm, s);
   combine(ctx, out, t_main, D, c.data(), d.data(), 1, count, Lm, s);
 }
@@ -2753,8 +2754,8 @@ int shg_bfv_mul(shg_context* ctx, uint64_t* out, const uint64_t* a, const uint64
     // P/t * a_i (mod P) and (mod Q)
     bfv_scale_up(ctx, ac, X, a_aux, a_main, cc * 2, Lm, ls);
     // the tensor product mod Q and mod P
-    shg::launch_tensor(ctx->dev(), t_main, a_main, bc, cc, Lm, ls);
-    shg::launch_tensor(ctx->aux_dev(), t_aux, a_aux, b_aux, cc, K, ls);
+    shg::launch_tensor(ctx->dev().next(), t_main, a_main, bc, cc, Lm, ls);
+    shg::launch_tensor(ctx->aux_dev().next(), t_aux, a_aux, b_aux, cc, K, ls);
     // Q/t * tensor (mod Q)
     bfv_scale_reduce(ctx, out + (size_t)c0 * 3 * pm, t_main, t_aux, X, cc * 3, Lm, ls);
   }
@@ -2895,8 +2896,8 @@ extern "C" int shg_relin_apply_noalloc(shg_context* ctx, const shg_key* key,
     const int cc = std::min(C, count - c0);
     const uint64_t* src = ct + (size_t)c0 * 3 * Ln;
     shg::launch_intt_export(dv, X, src, 3, 2, 0, CtMap::identity(), cc, L, s);
-    shg::launch_keyswitch(dv, D, X, key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
-                          key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src, 3 * Ln,
+    shg::launch_keyswitch(dv.next(), D, X, key->d_digits, k, key->digit_flags, key->chunk,
+                          key->chunk_lazy, key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src, 3 * Ln,
                           CtMap::identity(), 0, 0, cc, L, s, shg::KeyTable{},
                           ks32_for(ctx, key, count, true));
   }

@@ -431,6 +431,7 @@ __global__ void k_substitute(uint64_t* out, const uint64_t* in, int power,
 // Two adjacent coefficients of ciphertexts blockIdx.y, + gridDim.y, ... per thread.
 __global__ void k_tensor(uint64_t* out, const uint64_t* a, const uint64_t* b, int count,
                          int log_n, int L, CtxDev c) {
+  after_previous();
   const size_t Ln = (size_t)L << log_n;
   const size_t r = ((size_t)blockIdx.x * blockDim.x + threadIdx.x) * 2;
   if (r >= Ln) return;
@@ -1132,7 +1133,7 @@ void launch_tensor(const CtxDev& c, uint64_t* out, const uint64_t* a,
   if (total == 0) return;
   LaunchScope scope_("tensor", s);
   const dim3 grid((unsigned)(((size_t)L * c.n / 2 + 255) / 256), std::min(count, 65535));
-  k_tensor<<<grid, 256, 0, s>>>(out, a, b, count, c.log_n, L, c);
+  launch_next(c.follows, k_tensor, grid, 256, 0, s, out, a, b, count, c.log_n, L, c);
 }
 
 void launch_tensor_intt(const CtxDev& c, uint64_t* out01, uint64_t* X,
@@ -1272,7 +1273,7 @@ void launch_modreduce_ntt(const CtxDev& c, uint64_t* out, uint64_t* Y,
   LaunchScope scope_("modreduce_lift", s);
   if (use_ntt4_mod(c)) {
     g_launch_count++;  // second phase kernel
-    launch4_modreduce_lift(c, out, Y, in, sc, count, L, s);
+    launch4_modreduce_lift(c.next(), out, Y, in, sc, count, L, s);
     return;
   }
 #define F(LN)                                                                 \

@@ -39,6 +39,14 @@ struct CtxDev {
   int narrow_q;               // every q below 2^45 (implies small_q)
   int lazy_inv;               // every q below 2^53 (implies small_q): four-step inverse phases
                               // skip their conditional subtractions
+  // launch_next of the first kernel of a transform, tensor product or key switch.
+  int follows = 0;
+  // For such a launch directly behind another kernel of the same call and stream.
+  CtxDev next() const {
+    CtxDev c = *this;
+    c.follows = 1;
+    return c;
+  }
 };
 
 // Per-digit description of a gadget key (RnsGadget::Decompose order,
@@ -154,6 +162,38 @@ struct LaunchScope {
     }
   }
 };
+
+// First statement of every kernel that launch_next starts: waits until the kernel
+// before it on the stream is complete and its stores are visible.
+__device__ __forceinline__ void after_previous() {
+  asm volatile("griddepcontrol.wait;" ::: "memory");
+}
+
+// Launch of a kernel that begins with after_previous().  With `follows` (a kernel of
+// this library went onto the stream just before, no event wait or copy) its CTAs
+// are placed once the last CTA before it has exited, without the drain and
+// launch between two kernels, about 2 us: at n = 2^14, six 45-bit primes, one
+// ct-mult+relin 48 -> 41 us, two 64 -> 51, two inverse NTTs 14.5 -> 12.4, four forward
+// 16.6 -> 12.6, one BFV product 146 -> 105; batches that fill the GPU for many waves are within 1 %.  No kernel
+// triggers its successor itself: at its start, the waiting CTAs crowd onto the SMs
+// that have room (two inverse NTTs 18.5 us) and hold slots that another lane
+// would use (250 rotations 2230 -> 2315 us); before its stores, k32_rows loses
+// more than the overlap gives (eight ct-mult+relin 117 us against 112).
+template <class... P, class... A>
+void launch_next(bool follows, void (*kern)(P...), dim3 grid, int threads, size_t smem,
+                 cudaStream_t s, const A&... args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3(threads);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = s;
+  cudaLaunchAttribute attr{};
+  attr.id = cudaLaunchAttributeProgrammaticStreamSerialization;
+  attr.val.programmaticStreamSerializationAllowed = 1;
+  cfg.attrs = &attr;
+  cfg.numAttrs = follows ? 1 : 0;
+  cudaLaunchKernelEx(&cfg, kern, P(args)...);
+}
 
 // Blocks for a grid-stride loop over `work` items (at most 16 per SM).
 int grid_for(size_t work, int threads);
@@ -373,7 +413,7 @@ struct ConvRef {
 
 void launch_switch_basis(const PrimeDev* primes, ConvRef conv, int ns, int nd,
                          const uint64_t* in, size_t in_stride, uint64_t* out,
-                         size_t out_stride, int count, int log_n, cudaStream_t s);
+                         size_t out_stride, int count, int log_n, cudaStream_t s, bool follows = false);
 
 // out_i = (a_i * c[i] - b_i * d[i]) mod q_i over [count][L][n] with c, d
 // Montgomery scalars per limb (ScaleAndReduce / ModReduceMsb combines).

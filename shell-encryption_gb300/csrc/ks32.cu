@@ -44,6 +44,7 @@ template <int LOG_N, bool LZ>
 __global__ void __launch_bounds__(K32<LOG_N>::THREADS, 768 / K32<LOG_N>::THREADS)
     k32_digit_cols(const uint64_t* X, const DigitDesc* digits, Ks32Digits first, int k, int L,
                    int nsplit, uint32_t* D, const __grid_constant__ W32 w) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using G = K32<LOG_N>;
   using C = typename G::C;
@@ -134,6 +135,7 @@ template <int LOG_N, bool LZ, int T, int NT>
 __global__ void __launch_bounds__(NT, 768 / NT)
     k32_rows(const uint32_t* D, const uint32_t* key, uint32_t* E, int k, int L, int count,
              const __grid_constant__ W32 w) {
+  after_previous();
   extern __shared__ __align__(16) uint32_t sm32[];
   constexpr int R = 1 << (LOG_N - 7), kLimbs = NT / 64;
   const int groups = (count + T - 1) / T;
@@ -263,6 +265,7 @@ __global__ void __launch_bounds__(NT, 768 / NT)
 template <int LOG_N, bool LZ>
 __global__ void __launch_bounds__(Ntt4<LOG_N>::COL_THREADS, 640 / Ntt4<LOG_N>::COL_THREADS)
     k32_crt_cols(const uint32_t* E, const Crt32* crt, int L, uint64_t* out, const __grid_constant__ W32 w, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = typename S::CC;
   __shared__ __align__(16) uint64_t smem[S::COLS << S::A];
@@ -395,7 +398,8 @@ void run_rows(const Ks32& ks, const uint32_t* D, uint32_t* E, int k, int L, int 
     if (bytes > 48 * 1024)
       cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, bytes);
     const int groups = (count + T - 1) / T;
-    kern<<<3 * (1 << (LOG_N - 7)) * groups, NT, bytes, s>>>(D, ks.key, E, k, L, count, ks.w);
+    launch_next(true, kern, 3 * (1 << (LOG_N - 7)) * groups, NT, bytes, s, D, ks.key, E, k, L,
+                count, ks.w);
   };
   using N192 = std::integral_constant<int, 192>;
   using N384 = std::integral_constant<int, 384>;
@@ -434,7 +438,8 @@ void launch_ks32(const CtxDev& c, const Ks32& ks, uint64_t* scratch, const uint6
     const long long ctas = (long long)count * L * G::TILES;                            \
     const int split = ctas >= 4LL * c.sms ? 1 : (ctas * 3 >= 2LL * c.sms ? 3 : 9);     \
     auto kern = ks.lazy ? k32_digit_cols<LN, LN <= 14> : k32_digit_cols<LN, false>;    \
-    kern<<<(int)(ctas * split), G::THREADS, 0, s>>>(X, digits, ks.first, k, L, split, D, ks.w); \
+    launch_next(c.follows, kern, (int)(ctas * split), G::THREADS, 0, s, X, digits, \
+                ks.first, k, L, split, D, ks.w);                                       \
   }
     SHG_DISPATCH32(c.log_n, F)
 #undef F
@@ -455,7 +460,8 @@ void launch_ks32(const CtxDev& c, const Ks32& ks, uint64_t* scratch, const uint6
   {                                                                                   \
     using S = Ntt4<LN>;                                                               \
     auto kern = ks.lazy ? k32_crt_cols<LN, LN <= 14> : k32_crt_cols<LN, false>;       \
-    kern<<<count * 2 * L * S::COL_TILES, S::COL_THREADS, 0, s>>>(E, ks.crt, L, Y, ks.w, c); \
+    launch_next(true, kern, count * 2 * L * S::COL_TILES, S::COL_THREADS, 0, s, E, ks.crt, L, Y, \
+                ks.w, c);                                                             \
   }
     SHG_DISPATCH32(c.log_n, F)
 #undef F

@@ -415,6 +415,7 @@ template <int LOG_N, bool LAZY, class Src, bool SMALL_IN = false>
 __global__ void __launch_bounds__(Ntt4<LOG_N>::COL_THREADS,
                                   65536 / (Ntt4<LOG_N>::COL_THREADS * 72))
     k4_fwd_cols(Src src, PrimeMap pm, uint64_t* buf, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = typename S::CC;
   extern __shared__ uint64_t smem[];
@@ -447,6 +448,7 @@ __global__ void __launch_bounds__(Ntt4<LOG_N>::COL_THREADS,
                                   (sizeof(DT) == 4 ? 6 : 5) * 128 / Ntt4<LOG_N>::COL_THREADS)
     k4_digit_cols_all(const uint64_t* X, const DigitDesc* digits, int k, int L, int need_lift,
                       uint64_t* D, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = typename S::CC;
   extern __shared__ uint64_t smem[];
@@ -515,6 +517,7 @@ __global__ void __maxnreg__(72)
                const uint64_t* ka, uint64_t* out, const uint64_t* base,
                size_t base_ct_elems, CtMap map, int base1_zero, int subst_power,
                int L, KeyTable kt, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = typename S::RC;
   extern __shared__ uint64_t smem[];
@@ -621,6 +624,7 @@ __global__ void __maxnreg__(56)
                 const uint64_t* ka, uint64_t* out, const uint64_t* base,
                 size_t base_ct_elems, CtMap map, int base1_zero, int subst_power,
                 int L, KeyTable kt, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = NttCore<S::B, 3>;
   extern __shared__ uint64_t smem[];
@@ -718,6 +722,7 @@ __global__ void __launch_bounds__(32 * W, MB)
     k4_ks_rows_warp(const uint64_t* buf, int k, const uint64_t* kb, const uint64_t* ka,
                     uint64_t* out, const uint64_t* base, size_t base_ct_elems, CtMap map,
                     int base1_zero, int subst_power, int L, KeyTable kt, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = NttCore<S::B, 2>;
   static_assert(C::T == 32 && C::E == 4 && C::P == 4, "32 threads x 4 values per row");
@@ -924,6 +929,7 @@ struct RowWork {
 template <int LOG_N, bool LAZY, class Dst, bool SHARE>
 __global__ void __launch_bounds__(32 * kRowWarps, 6)
     k4_fwd_rows(const uint64_t* buf, Dst dst, PrimeMap pm, int num, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = typename S::RC;
   __shared__ __align__(16) uint64_t smem[kRowBytes / 8];
@@ -987,6 +993,7 @@ __global__ void __launch_bounds__(32 * kRowWarps, 6)
 template <int LOG_N, bool LAZY, class Dst, int W, int DPI>
 __global__ void __launch_bounds__(32 * W)
     k4_fwd_rows_warp(const uint64_t* buf, Dst dst, PrimeMap pm, int num, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = NttCore<S::B, 2>;
   static_assert(C::T == 32 && C::E == 4 && C::P == 4, "32 threads x 4 values per row");
@@ -1054,6 +1061,7 @@ __global__ void __launch_bounds__(32 * W)
 template <int LOG_N, int INV, class Src, int W, int DPI>
 __global__ void __launch_bounds__(32 * W)
     k4_inv_rows_warp(Src src, PrimeMap pm, uint64_t* buf, int num, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = NttCore<S::B, 2>;
   static_assert(C::T == 32 && C::E == 4 && C::P == 4, "32 threads x 4 values per row");
@@ -1121,6 +1129,7 @@ __global__ void __launch_bounds__(32 * W)
 template <int LOG_N, int INV, class Src>
 __global__ void __launch_bounds__(Ntt4<LOG_N>::ROW_THREADS)
     k4_inv_rows(Src src, PrimeMap pm, uint64_t* buf, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = typename S::RC;
   extern __shared__ uint64_t smem[];
@@ -1171,6 +1180,7 @@ __global__ void __launch_bounds__(Ntt4<LOG_N>::ROW_THREADS)
 template <int LOG_N, int INV, class Dst>
 __global__ void __launch_bounds__(Ntt4<LOG_N>::COL_THREADS)
     k4_inv_cols(const uint64_t* buf, Dst dst, PrimeMap pm, CtxDev c) {
+  after_previous();
   using S = Ntt4<LOG_N>;
   using C = typename S::CC;
   extern __shared__ uint64_t smem[];
@@ -1217,7 +1227,8 @@ void fwd_rows4(const CtxDev& c, const uint64_t* buf, const Dst& dst, PrimeMap pm
   auto k2 = share ? (lazy ? k4_fwd_rows<LOG_N, true, Dst, true> : k4_fwd_rows<LOG_N, false, Dst, true>)
                   : (lazy ? k4_fwd_rows<LOG_N, true, Dst, false>
                           : k4_fwd_rows<LOG_N, false, Dst, false>);
-  k2<<<row_grid<LOG_N>(num, pm.L, share), 32 * kRowWarps, 0, s>>>(buf, dst, pm, num, c);
+  launch_next(true, k2, row_grid<LOG_N>(num, pm.L, share), 32 * kRowWarps, 0, s, buf, dst, pm,
+              num, c);
 }
 
 template <int LOG_N, class Src, class Dst>
@@ -1232,7 +1243,7 @@ void fwd4(const CtxDev& c, const Src& src, const Dst& dst, PrimeMap pm,
       if (small_in) k1 = k4_fwd_cols<LOG_N, LZ, Src, true>;
     }
     set_smem4(k1, S::COL_SMEM);
-    k1<<<num * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s>>>(src, pm, buf, c);
+    launch_next(c.follows, k1, num * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s, src, pm, buf, c);
   };
   if (c.small_q)
     cols(std::true_type{});
@@ -1254,13 +1265,14 @@ void inv4_mode(const CtxDev& c, const Src& src, const Dst& dst, PrimeMap pm,
     const int groups = pm.L * ((num / pm.L + DPI - 1) / DPI);
     auto k1 = k4_inv_rows_warp<LOG_N, INV, Src, W, DPI>;
     set_smem4(k1, W * DPI * (1 << S::B) * 8);
-    k1<<<groups * (1 << S::A) / W, 32 * W, W * DPI * (1 << S::B) * 8, s>>>(src, pm, buf, num, c);
+    launch_next(c.follows, k1, groups * (1 << S::A) / W, 32 * W, W * DPI * (1 << S::B) * 8, s, src,
+                pm, buf, num, c);
   } else {
     auto k1 = k4_inv_rows<LOG_N, INV, Src>;
     set_smem4(k1, S::ROW_SMEM);
-    k1<<<num * S::ROW_TILES, S::ROW_THREADS, S::ROW_SMEM, s>>>(src, pm, buf, c);
+    launch_next(c.follows, k1, num * S::ROW_TILES, S::ROW_THREADS, S::ROW_SMEM, s, src, pm, buf, c);
   }
-  k2<<<num * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s>>>(buf, dst, pm, c);
+  launch_next(true, k2, num * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s, buf, dst, pm, c);
 }
 
 template <int LOG_N, class Src, class Dst>
@@ -1356,7 +1368,8 @@ void launch4_digit_cols(const CtxDev& c, uint64_t* D, const uint64_t* X,
     auto k1 = c.small_q ? k4_digit_cols_all<LN, true, uint32_t>                 \
                         : k4_digit_cols_all<LN, false, uint32_t>;               \
     set_smem4(k1, S::COL_SMEM);                                                 \
-    k1<<<count * k * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s>>>(X, digits, k, L, 0, D, c); \
+    launch_next(c.follows, k1, count * k * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s, X, \
+                digits, k, L, 0, D, c);                                                 \
   }
     SHG_DISPATCH4(c.log_n, F)
 #undef F
@@ -1373,7 +1386,8 @@ void launch4_digit_cols(const CtxDev& c, uint64_t* D, const uint64_t* X,
       k1 = c.small_q ? k4_fwd_cols<LN, true, FwdSrcDigit<LN>, true>             \
                      : k4_fwd_cols<LN, false, FwdSrcDigit<LN>, true>;           \
     set_smem4(k1, S::COL_SMEM);                                                 \
-    k1<<<count * k * L * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s>>>(       \
+    launch_next(                                                                \
+        c.follows, k1, count * k * L * S::COL_TILES, S::COL_THREADS, S::COL_SMEM, s, \
         src, PrimeMap{0, 1, L}, D, c);                                          \
   }
   SHG_DISPATCH4(c.log_n, F)
@@ -1401,7 +1415,8 @@ void launch4_ks_rows(const CtxDev& c, const uint64_t* D, int k, int chunk,
     if (c.narrow_q) kern = k4_ks_rows_warp<LN, true, kKsWarpRows, 4, kKsWarpDigits, true>; \
     const int smem = kKsWarpRows * kKsWarpDigits * 128 * 8;                     \
     set_smem4(kern, smem);                                                      \
-    kern<<<count * L * ((1 << (LN - 7)) / kKsWarpRows), 32 * kKsWarpRows, smem, s>>>( \
+    launch_next(                                                                \
+        true, kern, count * L * ((1 << (LN - 7)) / kKsWarpRows), 32 * kKsWarpRows, smem, s, \
         D, k, kb, ka, out, base, base_ct_elems, map, base1_zero, subst_power, L, kt, c); \
   }
     SHG_DISPATCH4(c.log_n, F)
@@ -1415,7 +1430,8 @@ void launch4_ks_rows(const CtxDev& c, const uint64_t* D, int k, int chunk,
     auto kern = c.small_q ? k4_ks_rows8<LN, true> : k4_ks_rows8<LN, false>;     \
     const int smem = k * (1 << S::B) * 8;                                       \
     set_smem4(kern, smem);                                                      \
-    kern<<<count * L * (1 << S::A), k * 16, smem, s>>>(                         \
+    launch_next(                                                                \
+        true, kern, count * L * (1 << S::A), k * 16, smem, s,                      \
         D, k, chunk, kb, ka, out, base, base_ct_elems, map, base1_zero,         \
         subst_power, L, kt, c);                                                 \
   }
@@ -1431,7 +1447,8 @@ void launch4_ks_rows(const CtxDev& c, const uint64_t* D, int k, int chunk,
     const int threads = R * k * S::RC::T;                                       \
     const int smem = R * k * (1 << S::B) * 8;                                   \
     set_smem4(kern, smem);                                                      \
-    kern<<<count * L * ((1 << S::A) / R), threads, smem, s>>>(                  \
+    launch_next(                                                                \
+        true, kern, count * L * ((1 << S::A) / R), threads, smem, s,               \
         D, k, R, chunk, kb, ka, out, base, base_ct_elems, map, base1_zero,      \
         subst_power, L, kt, c);                                                 \
   }
@@ -1453,7 +1470,8 @@ void launch4_rows_add(const CtxDev& c, const uint64_t* buf, uint64_t* out, const
     const int groups = (2 * count + dpi - 1) / dpi;                                  \
     auto kern = dpi == 1 ? k4_fwd_rows_warp<LN, true, Dst, W, 1>                     \
                          : k4_fwd_rows_warp<LN, true, Dst, W, kRowsWarpDpi>;         \
-    kern<<<L * groups * (1 << (LN - 7)) / W, 32 * W, W * dpi * 128 * 8, s>>>(        \
+    launch_next(                                                                     \
+        true, kern, L * groups * (1 << (LN - 7)) / W, 32 * W, W * dpi * 128 * 8, s,     \
         buf, dst, PrimeMap{0, 1, L}, 2 * count * L, c);                              \
   }
   SHG_DISPATCH4(c.log_n, F)
