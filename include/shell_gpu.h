@@ -177,7 +177,9 @@ int shg_ct_tensor(shg_context* ctx, uint64_t* out, const uint64_t* a,
  * the Galois power for an RnsGaloisKey (CreateFromKeyComponents,
  * rns/rns_galois_key.cc:183-202).  A single-modulus RelinearizationKey /
  * GaloisKey part is the num_limbs == 1 case (relinearization_key.cc:99-141;
- * galois_key.h:43-111). */
+ * galois_key.h:43-111).  Keys whose digits have at most 26 bits also keep a
+ * 32-bit form for batched key switches (device memory 2.5 times that of the
+ * rows); where it cannot be allocated, batches use the rows. */
 int shg_key_create(shg_context* ctx, int num_limbs, const int* log_bs,
                    int power, const uint64_t* key_b, const uint64_t* key_a,
                    shg_key** out);
