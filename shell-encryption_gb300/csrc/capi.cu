@@ -2356,9 +2356,13 @@ static size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 // Scratch of the side-by-side sampler, 0 where the sequential one runs: it
 // pays while less than one of a ciphertext's uniform words is rejected on
 // average (half of a 45-bit prime's ciphertexts in 200 have one, all of a prime's
-// just above a power of two have n).
+// just above a power of two have n).  Up to 4096 words of a ciphertext are a few
+// passes of one CTA, shorter than the second launch (sequential against side by
+// side, us: n = 2^11, one limb, 40 / 400 / 2500 ciphertexts 14 / 23 / 79 against
+// 19 / 30 / 85, n = 2^12 20 / 35 / 136 against 24 / 41 / 142; above, 6144 words 400 /
+// 2500 39 / 159 against 39 / 152, 8192 words 1000 92 against 79).
 static size_t reject_bytes(const shg_context* ctx, int L, int count) {
-  if (ctx->n < 64) return 0;
+  if ((size_t)ctx->n * L <= 4096) return 0;
   double expected = 0;
   for (int l = 0; l < L; ++l)
     expected += ctx->n * (1.0 - (double)ctx->hp[l].q / std::ldexp(1.0, ctx->hp[l].log_q));
