@@ -177,9 +177,17 @@ int shg_ct_tensor(shg_context* ctx, uint64_t* out, const uint64_t* a,
  * the Galois power for an RnsGaloisKey (CreateFromKeyComponents,
  * rns/rns_galois_key.cc:183-202).  A single-modulus RelinearizationKey /
  * GaloisKey part is the num_limbs == 1 case (relinearization_key.cc:99-141;
- * galois_key.h:43-111).  Keys whose digits have at most 26 bits also keep a
- * 32-bit form for batched key switches (device memory 2.5 times that of the
- * rows); where it cannot be allocated, batches use the rows. */
+ * galois_key.h:43-111).
+ *
+ * Keys of at least four limbs at n = 2^12 .. 2^15 with primes below 2^57 and at
+ * most 128 digits of at most 26 bits, all below every prime, have a 32-bit form
+ * beside the rows: 1.5 times their size.  The first batch with this one key that
+ * is large enough to gain from it makes the form (with another 1.25 times the
+ * rows for the time of the making) while a quarter of the device's memory stays
+ * free; batches with one key per member, captures and shg_relin_apply_noalloc
+ * never make it.  It goes back when an allocation of this library finds the
+ * device full, but not once a captured call has used it.  Results are the same
+ * with and without. */
 int shg_key_create(shg_context* ctx, int num_limbs, const int* log_bs,
                    int power, const uint64_t* key_b, const uint64_t* key_a,
                    shg_key** out);
@@ -192,7 +200,7 @@ int shg_key_num_limbs(const shg_key* key);
 int shg_key_log_bs(const shg_key* key, int* log_bs, int max);
 int shg_key_power(const shg_key* key);
 shg_context* shg_key_context(const shg_key* key);
-/* Device bytes held by the key. */
+/* Device bytes of the key: its rows and, made or not, its 32-bit form. */
 size_t shg_key_device_bytes(const shg_key* key);
 
 /* RnsRelinKey::ApplyTo for degree-2 ciphertexts

@@ -221,7 +221,10 @@ int plan(shg_batch* b) {
   }
   for (int i = 0; i < kStreams; ++i) {
     if (b->arena_elems[i] == 0) continue;
-    cudaError_t e = cudaMalloc(&b->arena[i], b->arena_elems[i] * sizeof(uint64_t));
+    const size_t bytes = b->arena_elems[i] * sizeof(uint64_t);
+    cudaError_t e = cudaMalloc(&b->arena[i], bytes);
+    if (e == cudaErrorMemoryAllocation && shg::give_back_key_forms())
+      e = cudaMalloc(&b->arena[i], bytes);
     if (e != cudaSuccess) {
       cudaGetLastError();
       b->release_plan();

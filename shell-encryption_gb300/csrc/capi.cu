@@ -162,6 +162,17 @@ int set_error(int code, const std::string& msg) { return fail(code, msg); }
 // Context and key objects
 // ---------------------------------------------------------------------------
 
+namespace {
+// cudaMalloc for the library's own buffers and shg_device_alloc: where memory is
+// short, once more after the keys' 32-bit forms went back.  held: the context
+// whose mu the caller holds.
+cudaError_t device_malloc(void** p, size_t bytes, shg_context* held = nullptr);
+template <class T>
+cudaError_t device_malloc(T** p, size_t bytes, shg_context* held = nullptr) {
+  return device_malloc(reinterpret_cast<void**>(p), bytes, held);
+}
+}  // namespace
+
 struct shg_context {
   int log_n = 0, n = 0, L = 0;
   int K = 0;  // auxiliary primes (BFV basis extension), after the L main ones
@@ -209,7 +220,7 @@ struct shg_context {
   cudaStream_t io_lanes[kMaxKsLanes] = {};
   std::mutex io_mu;
   // Auxiliary primes of the 32-bit key switch (ks32.cu), made with the first
-  // key that uses them: [0] below 2^30, [1] below 2^28 (lazy), with twiddles
+  // key that has that form: [0] below 2^30, [1] below 2^28 (lazy), with twiddles
   // [2][3][n] and one Crt32 per main limb.
   struct Set32 {
     shg::W32 w{};
@@ -242,7 +253,7 @@ struct shg_context {
       ws = nullptr;
       ws_bytes = 0;
     }
-    cudaError_t e = cudaMalloc(&ws, bytes);
+    cudaError_t e = device_malloc(&ws, bytes, this);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(SHG_RESOURCE_EXHAUSTED,
@@ -265,12 +276,60 @@ struct shg_key {
   int digit_flags = 0;  // shg::digit_flags(need_lift, largest log_b)
   int chunk = 1;       // digits per REDC for canonical digit transforms
   int chunk_lazy = 1;  // the same for lazily reduced ones (below 62 q)
-  shg::Ks32 ks32;           // the key in the 32-bit auxiliary primes, if it has that form
-  uint32_t* d_key32 = nullptr;
-  size_t bytes = 0;
+  // The key in the 32-bit auxiliary primes, under ctx->mu: its shape from the
+  // key's creation on (bytes 0: it has none), the words (ks.key) made by the
+  // first batch that takes them and given back when memory runs short.
+  struct Form32 {
+    shg::Ks32 ks;
+    uint32_t* words = nullptr;
+    size_t bytes = 0;
+    int wait = 0;           // calls before another attempt, after one without room
+    bool captured = false;  // a graph may hold the words: they stay
+  };
+  mutable Form32 form32;
+  size_t bytes = 0;  // rows, digits and the 32-bit form
 };
 
 namespace {
+
+// Keys whose 32-bit words are on a device.  Locked after a context's mu, never
+// before one (give_back_forms only tries those).
+std::mutex g_forms_mu;
+std::vector<const shg_key*> g_forms;
+
+void drop_form(const shg_key* key) {
+  cudaFree(key->form32.words);
+  key->form32.words = nullptr;
+  key->form32.ks.key = nullptr;
+}
+
+// Frees the words of every key of the current device, but for those that a graph
+// may hold and those of contexts that another thread is in.  True if it freed any.
+bool give_back_forms(shg_context* held) {
+  cudaGetLastError();  // of the allocation that the caller tries again
+  int device = -1;
+  if (cudaGetDevice(&device) != cudaSuccess) return false;
+  std::lock_guard<std::mutex> list(g_forms_mu);
+  const size_t before = g_forms.size();
+  auto gone = [&](const shg_key* key) {
+    shg_context* ctx = key->ctx;
+    if (ctx->device != device) return false;
+    std::unique_lock<std::mutex> lock(ctx->mu, std::defer_lock);
+    if (ctx != held && !lock.try_lock()) return false;
+    // kernels that read the words
+    if (key->form32.captured || cudaDeviceSynchronize() != cudaSuccess) return false;
+    drop_form(key);
+    return true;
+  };
+  g_forms.erase(std::remove_if(g_forms.begin(), g_forms.end(), gone), g_forms.end());
+  return g_forms.size() < before;
+}
+
+cudaError_t device_malloc(void** p, size_t bytes, shg_context* held) {
+  cudaError_t e = cudaMalloc(p, bytes);
+  if (e != cudaErrorMemoryAllocation || !give_back_forms(held)) return e;
+  return cudaMalloc(p, bytes);
+}
 
 bool aligned16(const void* p) { return ((uintptr_t)p & 15) == 0; }
 
@@ -311,23 +370,15 @@ int launch_status(const char* what) {
   return SHG_OK;
 }
 
-// The key's 32-bit form if a key switch of `count` ciphertexts with this one
-// key should use it (ks32.cu), else an empty one.  Counted in 64-bit transforms
-// of n, it saves k L of them and costs 0.45 of one per 32-bit transform (3 k + 6 L)
-// and 2 L; two more launches need a saving of about 1.75 M coefficients (measured
-// break-even: n = 2^14, 6 limbs between 1 and 2 ciphertexts (49.7 / 53.6 and
-// 69.8 / 63.7 us), 4 limbs at 6 (83.3 / 84.0); n = 2^13, 4 limbs between 8 and 16
-// (61.7 / 65.5 and 97.6 / 92.4); n = 2^12, 12 limbs at 2 (71.6 / 74.1)).
-const shg::Ks32& ks32_for(const shg_context* ctx, const shg_key* key, int count, bool one_key) {
-  static const shg::Ks32 none;
-  const CtxDev c = ctx->dev();
-  if (!key->ks32.key || !one_key || !c.ks_fused || (c.log_n < c.ntt4_plain_min && c.log_n <= 14))
-    return none;
-  const double k = key->k, L = key->L;
-  const double saved = k * L - 0.45 * (3 * k + 6 * L) - 2 * L;
-  return saved * count * ctx->n >= 1.75e6 ? key->ks32 : none;
-}
-// Digit scratch of one ciphertext of a key switch through that form or without.
+}  // namespace
+
+namespace shg {
+bool give_back_key_forms() { return give_back_forms(nullptr); }
+}  // namespace shg
+
+namespace {
+
+// Digit scratch of one ciphertext of a key switch through the 32-bit form or without.
 // Workspaces hold the larger need of the two, so that a call of fewer
 // ciphertexts (which may take the other form) never needs more than one of more.
 size_t ks_scratch_bytes(const shg_context* ctx, const shg_key* key, const shg::Ks32& ks32) {
@@ -637,6 +688,15 @@ int shg_context_create_with_aux(int log_n, const uint64_t* qs, int num_qs, const
 
 void shg_context_destroy(shg_context* ctx) {
   if (!ctx) return;
+  {
+    std::lock_guard<std::mutex> list(g_forms_mu);
+    auto gone = [&](const shg_key* key) {
+      if (key->ctx != ctx) return false;
+      drop_form(key);
+      return true;
+    };
+    g_forms.erase(std::remove_if(g_forms.begin(), g_forms.end(), gone), g_forms.end());
+  }
   cudaFree(ctx->d_conv);
   cudaFree(ctx->d_primes);
   cudaFree(ctx->d_tw_fwd);
@@ -1034,8 +1094,7 @@ int make_set32(shg_context* ctx, int lazy) {
   return SHG_OK;
 }
 
-// Gives the key (already on the device) its 32-bit form where launch_ks32 can
-// and should use it:
+// Plans the key's 32-bit form where launch_ks32 can and should use it:
 //  - n = 2^12 .. 2^15 (its transforms) and at least kKs32MinLimbs limbs: with
 //    few limbs the reconstruction costs more than the digit transforms it saves;
 //  - plain digits of at most 26 bits (below every auxiliary prime, no lift);
@@ -1045,9 +1104,8 @@ int make_set32(shg_context* ctx, int lazy) {
 //    2^28 (n <= 2^14: at most 7 levels per phase) or else those below 2^30;
 //  - at most 128 digits (one row of each in shared memory) and scratch no
 //    larger than the general path's digit transforms.
-// Without device memory for it the key works as it is.
 constexpr int kKs32MinLimbs = 4;
-void make_key32(shg_context* ctx, shg_key* key, const std::vector<DigitDesc>& dd) {
+void plan_form32(shg_context* ctx, shg_key* key, const std::vector<DigitDesc>& dd) {
   const int L = key->L, k = key->k, log_n = ctx->log_n;
   const size_t n = ctx->n;
   if (log_n < 12 || log_n > 15 || L < kKs32MinLimbs || key->digit_flags != 0) return;
@@ -1073,45 +1131,106 @@ void make_key32(shg_context* ctx, shg_key* key, const std::vector<DigitDesc>& dd
     }
   }
   if (lazy < 0 || make_set32(ctx, lazy) != SHG_OK) return;
-  const size_t elems = (size_t)k * L * n;
-  uint64_t* rows = nullptr;
-  uint32_t *tmp = nullptr, *key32 = nullptr;
-  cudaError_t e = cudaMalloc(&rows, elems * sizeof(uint64_t));
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, 3 * elems * sizeof(uint32_t));
+  const shg_context::Set32& set = ctx->set32[lazy];
+  shg_key::Form32& f = key->form32;
   // the row kernel fetches a few digits ahead of the last row's end
-  const size_t key_words = 6 * elems + (size_t)shg::kKs32PadDigits * L * 256;
-  if (e == cudaSuccess) e = cudaMalloc(&key32, key_words * sizeof(uint32_t));
+  f.bytes = (6 * (size_t)k * L * n + (size_t)shg::kKs32PadDigits * L * 256) * sizeof(uint32_t);
+  f.ks.crt = set.d_crt;
+  f.ks.lazy = lazy;
+  f.ks.w = set.w;
+  int j = 0;
+  for (int l = 0; l < L; ++l) {
+    f.ks.first.j[l] = (short)j;
+    while (j < k && dd[j].src_limb == l) ++j;
+  }
+  f.ks.first.j[L] = (short)j;
+  key->bytes += f.bytes;
+}
+
+// Makes the words of the key's form (under ctx->mu; the calling stream is not
+// being captured) while a quarter of the device's memory stays free, else leaves
+// the key to its rows and looks again 256 calls later.  On a stream of its own and
+// in relaxed capture mode, so that a capture of another stream is not disturbed.
+// 0.57 ms for six limbs at n = 2^14 (42 MB beside 28 MB of rows), 2.1 ms for twelve
+// at n = 2^15 (340 beside 226 MB), once per key.
+void make_form32(shg_context* ctx, const shg_key* key) {
+  shg_key::Form32& f = key->form32;
+  if (f.wait > 0) {
+    --f.wait;
+    return;
+  }
+  f.wait = 256;
+  const int L = key->L, k = key->k;
+  const size_t elems = (size_t)k * L * ctx->n;
+  const size_t row_bytes = elems * sizeof(uint64_t), tmp_bytes = 3 * elems * sizeof(uint32_t);
+  cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  uint64_t* rows = nullptr;
+  uint32_t *tmp = nullptr, *words = nullptr;
+  cudaStream_t s = nullptr;
+  size_t room = 0, total = 0;
+  cudaError_t e = cudaMemGetInfo(&room, &total);
+  if (e == cudaSuccess && room < f.bytes + row_bytes + tmp_bytes + total / 4)
+    e = cudaErrorMemoryAllocation;
+  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
+  if (e == cudaSuccess) e = cudaMalloc(&rows, row_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&tmp, tmp_bytes);
+  if (e == cudaSuccess) e = cudaMalloc(&words, f.bytes);
   if (e == cudaSuccess) {
-    const shg_context::Set32& set = ctx->set32[lazy];
-    const CtxDev dv = ctx->dev();
     for (int c = 0; c < 2; ++c) {
       // the stored rows carry 2^64 mod q: the export scaling takes it off
-      shg::launch_ntt_inv(dv, c ? key->ka : key->kb, rows, k * L, L, 1, 0);
-      shg::launch_ks32_key(dv, set.w, rows, tmp, k, L, c, key32, 0);
+      shg::launch_ntt_inv(ctx->dev(), c ? key->ka : key->kb, rows, k * L, L, 1, s);
+      shg::launch_ks32_key(ctx->dev(), f.ks.w, rows, tmp, k, L, c, words, s);
     }
-    e = cudaDeviceSynchronize();
+    e = cudaGetLastError();
+    const cudaError_t done = cudaStreamSynchronize(s);
+    if (e == cudaSuccess) e = done;
   }
   cudaFree(rows);
   cudaFree(tmp);
-  if (e != cudaSuccess) {
+  if (s) cudaStreamDestroy(s);
+  if (e == cudaSuccess) {
+    f.words = words;
+    f.ks.key = words;
+    f.wait = 0;
+    std::lock_guard<std::mutex> list(g_forms_mu);
+    g_forms.push_back(key);
+  } else {
     cudaGetLastError();
-    cudaFree(key32);
-    return;
+    cudaFree(words);
   }
-  const shg_context::Set32& set = ctx->set32[lazy];
-  key->d_key32 = key32;
-  key->bytes += key_words * sizeof(uint32_t);
-  key->ks32.key = key32;
-  key->ks32.crt = set.d_crt;
-  key->ks32.lazy = lazy;
-  key->ks32.w = set.w;
-  int j = 0;
-  for (int l = 0; l < L; ++l) {
-    key->ks32.first.j[l] = (short)j;
-    while (j < k && dd[j].src_limb == l) ++j;
-  }
-  key->ks32.first.j[L] = (short)j;
+  cudaThreadExchangeStreamCaptureMode(&mode);
 }
+
+// The key's 32-bit form if a key switch of `count` ciphertexts with this one
+// key should use it (ks32.cu), else an empty one.  Counted in 64-bit transforms
+// of n, it saves k L of them and costs 0.45 of one per 32-bit transform (3 k + 6 L)
+// and 2 L; two more launches need a saving of about 1.75 M coefficients (measured
+// break-even: n = 2^14, 6 limbs between 1 and 2 ciphertexts (49.7 / 53.6 and
+// 69.8 / 63.7 us), 4 limbs at 6 (83.3 / 84.0); n = 2^13, 4 limbs between 8 and 16
+// (61.7 / 65.5 and 97.6 / 92.4); n = 2^12, 12 limbs at 2 (71.6 / 74.1)).
+//
+// `make`: the call may make the words; a capture of s takes them only if they are
+// there.  Keys that only multi-key batches use thus never hold them.  Under ctx->mu.
+const shg::Ks32& ks32_for(shg_context* ctx, const shg_key* key, int count, bool one_key,
+                          cudaStream_t s, bool make = true) {
+  static const shg::Ks32 none;
+  const CtxDev c = ctx->dev();
+  shg_key::Form32& f = key->form32;
+  if (!f.bytes || !one_key || !c.ks_fused || (c.log_n < c.ntt4_plain_min && c.log_n <= 14))
+    return none;
+  const double k = key->k, L = key->L;
+  const double saved = k * L - 0.45 * (3 * k + 6 * L) - 2 * L;
+  if (saved * count * ctx->n < 1.75e6) return none;
+  cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+  const bool captured = cudaStreamIsCapturing(s, &cap) != cudaSuccess ||
+                        cap != cudaStreamCaptureStatusNone;
+  if (!f.words && make && !captured) make_form32(ctx, key);
+  if (!f.words) return none;
+  f.captured |= captured;
+  return f.ks;
+}
+
 
 }  // namespace
 
@@ -1168,9 +1287,9 @@ int shg_key_create(shg_context* ctx, int num_limbs, const int* log_bs,
                                                              (~(uint64_t)0) / (62 * qmax)));
   const size_t elems = (size_t)key->k * num_limbs * ctx->n;
   key->bytes = 2 * elems * sizeof(uint64_t) + dd.size() * sizeof(DigitDesc);
-  cudaError_t e = cudaMalloc(&key->kb, elems * sizeof(uint64_t));
-  if (e == cudaSuccess) e = cudaMalloc(&key->ka, elems * sizeof(uint64_t));
-  if (e == cudaSuccess) e = cudaMalloc(&key->d_digits, dd.size() * sizeof(DigitDesc));
+  cudaError_t e = device_malloc(&key->kb, elems * sizeof(uint64_t));
+  if (e == cudaSuccess) e = device_malloc(&key->ka, elems * sizeof(uint64_t));
+  if (e == cudaSuccess) e = device_malloc(&key->d_digits, dd.size() * sizeof(DigitDesc));
   if (e == cudaSuccess)
     e = cudaMemcpy(key->kb, key_b, elems * sizeof(uint64_t), cudaMemcpyDefault);
   if (e == cudaSuccess)
@@ -1200,16 +1319,20 @@ int shg_key_create(shg_context* ctx, int num_limbs, const int* log_bs,
     shg_key_destroy(key);
     return cuda_fail(e, "key conversion");
   }
-  make_key32(ctx, key, dd);
+  plan_form32(ctx, key, dd);
   *out = key;
   return SHG_OK;
 }
 
 void shg_key_destroy(shg_key* key) {
   if (!key) return;
+  {
+    std::lock_guard<std::mutex> list(g_forms_mu);
+    g_forms.erase(std::remove(g_forms.begin(), g_forms.end(), key), g_forms.end());
+  }
+  drop_form(key);
   cudaFree(key->kb);
   cudaFree(key->ka);
-  cudaFree(key->d_key32);
   cudaFree(key->d_digits);
   delete key;
 }
@@ -1241,6 +1364,34 @@ struct KsArgs {
 int upload_key_table(const shg_key* const* keys, int count, int stride, int offset,
                      const uint64_t** dst, shg::KeyTable* out, cudaStream_t s);
 
+// Form, chunks and lanes of a batched key switch, its scratch made ready: x_per_ct
+// bytes per ciphertext of a chunk beside the digit scratch and `fixed` bytes beside
+// the chunks; budget and set_max as in ks_chunk.  Under ctx->mu.
+struct KsPlan {
+  const shg::Ks32* ks32;
+  size_t per_ct;
+  int C;
+};
+int plan_ks(KsLanes& lanes, const shg_key* key, int count, bool one_key, size_t x_per_ct,
+            size_t fixed, size_t budget, int set_max, KsPlan* p) {
+  shg_context* ctx = lanes.ctx;
+  const size_t plain = x_per_ct + ks_scratch_bytes(ctx, key, shg::Ks32{});
+  const int C_plain = ks_chunk(ctx, plain, count, budget, set_max);
+  for (bool make = true;; make = false) {
+    p->ks32 = &ks32_for(ctx, key, count, one_key, lanes.s, make);
+    p->per_ct = x_per_ct + ks_scratch_bytes(ctx, key, *p->ks32);
+    p->C = ks_chunk(ctx, p->per_ct, count, budget, set_max);
+    const bool form = p->ks32->key != nullptr;
+    int st = lanes.open((count + p->C - 1) / p->C);
+    if (st) return st;
+    const size_t need = std::max(
+        lanes.n * p->per_ct * p->C, lanes.lanes_of((count + C_plain - 1) / C_plain) * plain * C_plain);
+    if ((st = ctx->ensure_ws(need + fixed))) return st;
+    // the workspace may have taken the form's memory: `need` holds the other layout
+    if (!form || p->ks32->key) return SHG_OK;
+  }
+}
+
 // Gadget key switch of component a.comp of `count` ciphertexts; with `keys`,
 // member i uses keys[i] (same gadget shape as `key`).
 int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
@@ -1248,27 +1399,17 @@ int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
               const shg_key* const* keys = nullptr) {
   const int L = key->L, n = ctx->n, k = key->k;
   const size_t Ln = (size_t)L * n;
-  const shg::Ks32& ks32 = ks32_for(ctx, key, count, keys == nullptr);
-  const size_t d_per_ct = ks_scratch_bytes(ctx, key, ks32);
-  const size_t per_ct = Ln * sizeof(uint64_t) + d_per_ct;
-  const size_t per_ct_plain =
-      Ln * sizeof(uint64_t) + ks_scratch_bytes(ctx, key, shg::Ks32{});
-  constexpr size_t kBudget = (size_t)1 << 30;
-  const int C = ks_chunk(ctx, per_ct, count, kBudget, INT_MAX);
-  const int C_plain = ks_chunk(ctx, per_ct_plain, count, kBudget, INT_MAX);
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
   std::lock_guard<std::mutex> lock(ctx->mu);
-  // Each lane has its own X and D; two chunks side by side measured 17 % faster
-  // (250 rotations at n = 2^14, six limbs: 2971 -> 2268 us).
+  // Each lane has its own X and D; two chunks side by side take three quarters of
+  // the time (250 rotations at n = 2^14, six limbs: 2971 -> 2268 us).
   KsLanes lanes{ctx, s};
-  const int nchunks = (count + C - 1) / C;
-  int st = lanes.open(nchunks);
+  KsPlan p;
+  int st = plan_ks(lanes, key, count, keys == nullptr, Ln * sizeof(uint64_t), tab_bytes,
+                   (size_t)1 << 30, INT_MAX, &p);
   if (st) return st;
-  const size_t lane_bytes = per_ct * C;
-  const size_t need =
-      std::max(lanes.n * lane_bytes, lanes.lanes_of((count + C_plain - 1) / C_plain) *
-                                         (per_ct_plain * C_plain));
-  if ((st = ctx->ensure_ws(need + tab_bytes))) return st;
+  const int C = p.C, nchunks = (count + C - 1) / C;
+  const size_t lane_bytes = p.per_ct * C;
   shg::KeyTable table;
   if (keys && (st = upload_key_table(keys, count, 1, 0,
                                      reinterpret_cast<const uint64_t**>(
@@ -1289,7 +1430,7 @@ int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
     shg::launch_keyswitch(dv.next(), D, X, key->d_digits, k, key->digit_flags, key->chunk,
                           key->chunk_lazy, key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src,
                           (size_t)a.ncomp * Ln, CtMap::identity(), a.base1_zero,
-                          a.subst_power, cc, L, lanes.stream(lane), kt, ks32);
+                          a.subst_power, cc, L, lanes.stream(lane), kt, *p.ks32);
   }
   if ((st = lanes.join())) return st;
   return launch_status("keyswitch");
@@ -1351,24 +1492,16 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
   // and the exported coefficients X of every degree-2 component.  Phase 2 in
   // chunks of the digit NTTs D and the key inner product.
   const size_t x_bytes = (size_t)count * Ln * sizeof(uint64_t);
-  const shg::Ks32& ks32 = ks32_for(ctx, key, count, keys == nullptr);
-  const size_t d_per_ct = ks_scratch_bytes(ctx, key, ks32);
-  auto chunk_of = [&](size_t per_ct) {
-    return ks_chunk(ctx, per_ct, count, (size_t)256 << 20, 16);
-  };
-  const int C = chunk_of(d_per_ct);
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
   std::lock_guard<std::mutex> lock(ctx->mu);
   // Chunks rotate over the lanes, each with its own digit scratch.
   KsLanes ks_lanes{ctx, s};
-  const int nchunks = (count + C - 1) / C;
-  if ((st = ks_lanes.open(nchunks))) return st;
-  const int lanes = ks_lanes.n;
-  const size_t d_plain = ks_scratch_bytes(ctx, key, shg::Ks32{});
-  const size_t need =
-      std::max(lanes * d_per_ct * C, ks_lanes.lanes_of((count + chunk_of(d_plain) - 1) / chunk_of(d_plain)) * d_plain *
-                   chunk_of(d_plain));
-  if ((st = ctx->ensure_ws(x_bytes + need + tab_bytes))) return st;
+  KsPlan p;
+  if ((st = plan_ks(ks_lanes, key, count, keys == nullptr, 0, x_bytes + tab_bytes,
+                    (size_t)256 << 20, 16, &p)))
+    return st;
+  const int C = p.C, nchunks = (count + C - 1) / C, lanes = ks_lanes.n;
+  const size_t d_per_ct = p.per_ct;
   uint64_t* X = ctx->ws;
   uint64_t* D0 = X + (size_t)count * Ln;
   shg::KeyTable kt;
@@ -1391,7 +1524,7 @@ int mul_relin_impl(shg_context* ctx, const shg_key* key, const shg_key* const* k
     shg::launch_keyswitch(lanes == 1 ? dv.next() : dv, D0 + lane * C * d_per_ct / 8,
                           X + (size_t)c0 * Ln, key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
                           key->kb, key->ka, o, o, 2 * Ln, CtMap::identity(), 0, 0, cc, L, ls,
-                          kc, ks32);
+                          kc, *p.ks32);
   }
   if ((st = ks_lanes.join())) return st;
   return launch_status("bgv_mul_relin");
@@ -1463,13 +1596,6 @@ int mul_relin_host_impl(shg_context* ctx, const shg_key* key, void* out_v, const
   const int S = ctx->host_slots;
   const size_t packed = wire ? 3 * (size_t)P * host_ct_pad : 0;
   const size_t slot = 3 * (size_t)P * ct_bytes + (size_t)P * Ln * sizeof(uint64_t) + packed;
-  const shg::Ks32& ks32 = ks32_for(ctx, key, count, true);
-  const size_t d_per_ct = ks_scratch_bytes(ctx, key, ks32);
-  auto chunk_of = [&](size_t per_ct) {
-    return ks_chunk(ctx, per_ct, P, (size_t)256 << 20, 16);
-  };
-  const int C = chunk_of(d_per_ct);
-  const size_t d_plain = ks_scratch_bytes(ctx, key, shg::Ks32{});
   const int lanes = std::max(1, std::min(ctx->ks_lanes, (int)shg_context::kMaxKsLanes));
   std::lock_guard<std::mutex> io_lock(ctx->io_mu);
   std::lock_guard<std::mutex> lock(ctx->mu);
@@ -1478,15 +1604,29 @@ int mul_relin_host_impl(shg_context* ctx, const shg_key* key, void* out_v, const
     cudaFree(ctx->io);
     ctx->io = nullptr;
     ctx->io_bytes = 0;
-    cudaError_t e = cudaMalloc(&ctx->io, S * slot);
+    cudaError_t e = device_malloc(&ctx->io, S * slot, ctx);
     if (e != cudaSuccess) {
       cudaGetLastError();
       return fail(SHG_RESOURCE_EXHAUSTED, "cannot reserve host-pipeline staging");
     }
     ctx->io_bytes = S * slot;
   }
-  if ((st = ctx->ensure_ws(lanes * std::max(C * d_per_ct, chunk_of(d_plain) * d_plain))))
-    return st;
+  const shg::Ks32* ks32;
+  size_t d_per_ct;
+  int C;
+  const size_t d_plain = ks_scratch_bytes(ctx, key, shg::Ks32{});
+  auto chunk_of = [&](size_t per_ct) {
+    return ks_chunk(ctx, per_ct, P, (size_t)256 << 20, 16);
+  };
+  for (bool make = true, form = true; form; make = false) {  // as in plan_ks
+    ks32 = &ks32_for(ctx, key, count, true, (cudaStream_t)stream, make);
+    d_per_ct = ks_scratch_bytes(ctx, key, *ks32);
+    C = chunk_of(d_per_ct);
+    form = ks32->key != nullptr;
+    if ((st = ctx->ensure_ws(lanes * std::max(C * d_per_ct, chunk_of(d_plain) * d_plain))))
+      return st;
+    if (ks32->key) break;
+  }
   uint64_t* D0 = ctx->ws;
   for (cudaStream_t& s : ctx->io_streams)
     if (!s) SHG_CUDA(cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking));
@@ -1588,7 +1728,7 @@ int mul_relin_host_impl(shg_context* ctx, const shg_key* key, void* out_v, const
       shg::launch_keyswitch(dv, D0 + lane * C * d_per_ct / 8, dx + (size_t)j * Ln,
                             key->d_digits, k, key->digit_flags, key->chunk, key->chunk_lazy,
                             key->kb, key->ka, o, o, 2 * Ln, CtMap::identity(), 0, 0, nc, L, ls,
-                            shg::KeyTable{}, ks32);
+                            shg::KeyTable{}, *ks32);
     }
     for (int lane = 0; lane < lanes; ++lane) {
       if (!used[lane]) continue;
@@ -1647,7 +1787,7 @@ int shg_key_components(const shg_key* key, uint64_t* key_b, uint64_t* key_a) {
   shg_context* ctx = key->ctx;
   const size_t elems = (size_t)key->k * key->L * ctx->n;
   uint64_t* tmp = nullptr;
-  cudaError_t e = cudaMalloc(&tmp, elems * sizeof(uint64_t));
+  cudaError_t e = device_malloc(&tmp, elems * sizeof(uint64_t));
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(SHG_RESOURCE_EXHAUSTED, "cannot reserve scratch for the key rows");
@@ -1679,8 +1819,8 @@ int shg_galois_key_compose(shg_context* ctx, const shg_key* key, const shg_key* 
   const size_t Ln = (size_t)L * ctx->n, bytes = Ln * sizeof(uint64_t);
   // The other key's rows as k ciphertexts (b_i, a_i), un-premultiplied.
   uint64_t *ct = nullptr, *res = nullptr;
-  cudaError_t e = cudaMalloc(&ct, 2 * k * bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&res, 2 * k * bytes);
+  cudaError_t e = device_malloc(&ct, 2 * k * bytes);
+  if (e == cudaSuccess) e = device_malloc(&res, 2 * k * bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     cudaFree(ct);
@@ -2114,7 +2254,7 @@ int shg_set_device(int device) {
   return SHG_OK;
 }
 int shg_device_alloc(size_t bytes, void** out) {
-  cudaError_t e = cudaMalloc(out, bytes);
+  cudaError_t e = device_malloc(out, bytes);
   if (e != cudaSuccess) {
     cudaGetLastError();
     return fail(SHG_RESOURCE_EXHAUSTED, std::string("cudaMalloc: ") + cudaGetErrorString(e));
@@ -2896,14 +3036,16 @@ extern "C" int shg_relin_apply_noalloc(shg_context* ctx, const shg_key* key,
   uint64_t* D = X + (size_t)C * Ln;
   cudaStream_t s = (cudaStream_t)stream;
   const CtxDev dv = ctx->dev();
+  std::lock_guard<std::mutex> lock(ctx->mu);
+  // the key's 32-bit form if an earlier batch made it
+  const shg::Ks32& ks32 = ks32_for(ctx, key, count, true, s, false);
   for (int c0 = 0; c0 < count; c0 += C) {
     const int cc = std::min(C, count - c0);
     const uint64_t* src = ct + (size_t)c0 * 3 * Ln;
     shg::launch_intt_export(dv, X, src, 3, 2, 0, CtMap::identity(), cc, L, s);
     shg::launch_keyswitch(dv.next(), D, X, key->d_digits, k, key->digit_flags, key->chunk,
                           key->chunk_lazy, key->kb, key->ka, out + (size_t)c0 * 2 * Ln, src, 3 * Ln,
-                          CtMap::identity(), 0, 0, cc, L, s, shg::KeyTable{},
-                          ks32_for(ctx, key, count, true));
+                          CtMap::identity(), 0, 0, cc, L, s, shg::KeyTable{}, ks32);
   }
   return launch_status("relin_apply_noalloc");
 }

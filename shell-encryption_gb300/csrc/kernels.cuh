@@ -456,6 +456,9 @@ void launch_scatter(uint64_t* const* dsts, const uint64_t* src, size_t elems, in
 // Sets this thread's last-error message (the C ABI's shg_last_error) and
 // returns `code`.
 int set_error(int code, const std::string& msg);
+// Frees the 32-bit forms of idle keys of the current device (capi.cu), for an
+// allocation that failed; true if that gave memory back.
+bool give_back_key_forms();
 
 // BGV encryption randomness from the ChaCha PRNG of seeds [count][32]
 // (RnsPolynomial::SampleUniform then SampleError): ciphertext p's uniform

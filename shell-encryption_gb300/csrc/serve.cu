@@ -217,6 +217,8 @@ void shg_server::launch(const GroupKey& gk, std::deque<uint64_t>& q, int stream)
   uint64_t* dev = nullptr;
   int st = SHG_OK;
   cudaError_t e = cudaMallocFromPoolAsync((void**)&dev, elems * 8, pool, s);
+  if (e == cudaErrorMemoryAllocation && shg::give_back_key_forms())
+    e = cudaMallocFromPoolAsync((void**)&dev, elems * 8, pool, s);
   if (e != cudaSuccess) {
     cudaGetLastError();
     finish(b.reqs, SHG_RESOURCE_EXHAUSTED, Clock::now());
