@@ -245,6 +245,12 @@ struct shg_context {
                   d_tw_inv + (size_t)L * n, nullptr, small_q, key_min(), ks_fused, sms,
                   ntt4_plain_min, ntt4_min, narrow_q, lazy_inv};
   }
+  // Whether a call on s can have `bytes` of scratch: a capture cannot grow it.
+  bool ws_fits(size_t bytes, cudaStream_t s) const {
+    if (bytes <= ws_bytes) return true;
+    cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
+    return cudaStreamIsCapturing(s, &cap) == cudaSuccess && cap == cudaStreamCaptureStatusNone;
+  }
   int ensure_ws(size_t bytes) {
     if (bytes <= ws_bytes) return SHG_OK;
     if (ws) {
@@ -1384,8 +1390,14 @@ int plan_ks(KsLanes& lanes, const shg_key* key, int count, bool one_key, size_t 
     const bool form = p->ks32->key != nullptr;
     int st = lanes.open((count + p->C - 1) / p->C);
     if (st) return st;
-    const size_t need = std::max(
+    size_t need = std::max(
         lanes.n * p->per_ct * p->C, lanes.lanes_of((count + C_plain - 1) / C_plain) * plain * C_plain);
+    if (!ctx->ws_fits(need + fixed, lanes.s)) {  // the lanes and chunks that it holds
+      const size_t room = ctx->ws_bytes > fixed ? ctx->ws_bytes - fixed : 0;
+      if (room < lanes.n * p->per_ct) lanes.n = 1;
+      p->C = std::max(1, (int)std::min<size_t>(p->C, room / (lanes.n * p->per_ct)));
+      need = lanes.n * p->per_ct * p->C;
+    }
     if ((st = ctx->ensure_ws(need + fixed))) return st;
     // the workspace may have taken the form's memory: `need` holds the other layout
     if (!form || p->ks32->key) return SHG_OK;
@@ -1962,8 +1974,8 @@ struct ExpandPlan {
   size_t bytes() const { return mono_bytes + lanes * per_member * C; }
 };
 
-ExpandPlan plan_expand(const shg_context* ctx, const shg_key* const* keys, int levels,
-                       int count, int lanes) {
+ExpandPlan plan_expand_on(const shg_context* ctx, const shg_key* const* keys, int levels,
+                          int count, int lanes) {
   ExpandPlan p;
   p.lanes = lanes;
   const int n = ctx->n;
@@ -1974,6 +1986,16 @@ ExpandPlan plan_expand(const shg_context* ctx, const shg_key* const* keys, int l
   p.C = std::max(1 << std::max(levels - 1, 0),
                  (int)std::min<size_t>((size_t)members_max, ((size_t)256 << 20) / p.per_member));
   return p;
+}
+
+// The plan on all lanes, on one where a capture has no scratch for more (`other`:
+// bytes beside the plan's).
+ExpandPlan plan_expand(const KsLanes& lanes, const shg_key* const* keys, int levels, int count,
+                       size_t other) {
+  const ExpandPlan p = plan_expand_on(lanes.ctx, keys, levels, count, lanes.n);
+  return lanes.ctx->ws_fits(p.bytes() + other, lanes.s)
+             ? p
+             : plan_expand_on(lanes.ctx, keys, levels, count, 1);
 }
 
 // ExpandCiphertext over `count` queries already placed at slot 0 of their
@@ -2070,9 +2092,9 @@ int pir_impl(shg_context* ctx, const shg_key* const* keys, bool per_query_keys, 
   std::lock_guard<std::mutex> lock(ctx->mu);
   KsLanes lanes{ctx, s};
   if ((st = lanes.open(group))) return st;
-  const ExpandPlan plan = plan_expand(ctx, keys, levels, group, lanes.n);
   const size_t blocks_bytes = (size_t)group * per_query_elems * sizeof(uint64_t);
   const size_t tab_bytes = per_query_keys ? 2 * (size_t)levels * count * sizeof(void*) : 0;
+  const ExpandPlan plan = plan_expand(lanes, keys, levels, group, blocks_bytes + tab_bytes);
   if ((st = ctx->ensure_ws(plan.bytes() + blocks_bytes + tab_bytes))) return st;
   uint64_t* blocks = ctx->ws + plan.bytes() / sizeof(uint64_t);
   std::vector<shg::KeyTable> tables(per_query_keys ? levels : 0);
@@ -2127,7 +2149,7 @@ int shg_oblivious_expand(shg_context* ctx, const shg_key* const* keys,
   std::lock_guard<std::mutex> lock(ctx->mu);
   KsLanes lanes{ctx, s};
   if ((st = lanes.open(count))) return st;
-  const ExpandPlan plan = plan_expand(ctx, keys, levels, count, lanes.n);
+  const ExpandPlan plan = plan_expand(lanes, keys, levels, count, 0);
   if ((st = ctx->ensure_ws(plan.bytes()))) return st;
   if ((st = run_expand(ctx, keys, levels, out, count, plan, ctx->ws, s))) return st;
   return launch_status("oblivious_expand");
@@ -2501,12 +2523,16 @@ static size_t round256(size_t b) { return (b + 255) & ~(size_t)255; }
 // side, us: n = 2^11, one limb, 40 / 400 / 2500 ciphertexts 14 / 23 / 79 against
 // 19 / 30 / 85, n = 2^12 20 / 35 / 136 against 24 / 41 / 142; above, 6144 words 400 /
 // 2500 39 / 159 against 39 / 152, 8192 words 1000 92 against 79).
-static size_t reject_bytes(const shg_context* ctx, int L, int count) {
+// A capture without scratch for the records beside `other` bytes takes the
+// sequential kernel.
+static size_t reject_bytes(const shg_context* ctx, int L, int count, size_t other,
+                           cudaStream_t s) {
   if ((size_t)ctx->n * L <= 4096) return 0;
   double expected = 0;
   for (int l = 0; l < L; ++l)
     expected += ctx->n * (1.0 - (double)ctx->hp[l].q / std::ldexp(1.0, ctx->hp[l].log_q));
-  return expected < 1 ? round256(count * shg::sample_reject_bytes()) : 0;
+  const size_t bytes = round256(count * shg::sample_reject_bytes());
+  return expected < 1 && ctx->ws_fits(other + bytes, s) ? bytes : 0;
 }
 
 int shg_sample_uniform_error(shg_context* ctx, uint64_t* a, uint64_t* e,
@@ -2522,7 +2548,7 @@ int shg_sample_uniform_error(shg_context* ctx, uint64_t* a, uint64_t* e,
   const size_t Ln = (size_t)L * ctx->n;
   std::lock_guard<std::mutex> lock(ctx->mu);
   const size_t err_bytes = round256((size_t)count * ctx->n * sizeof(int32_t));
-  const size_t rej_bytes = reject_bytes(ctx, L, count);
+  const size_t rej_bytes = reject_bytes(ctx, L, count, err_bytes, s);
   if ((st = ctx->ensure_ws(err_bytes + rej_bytes))) return st;
   int32_t* err = reinterpret_cast<int32_t*>(ctx->ws);
   const shg::CtxDev dev = ctx->dev();
@@ -2558,7 +2584,7 @@ int shg_bgv_encrypt(shg_context* ctx, uint64_t* out, const uint64_t* key,
   const int C = (int)std::max<size_t>(1, std::min<size_t>((size_t)count, want));
   const size_t err_bytes = round256((size_t)count * n * sizeof(int32_t));
   std::lock_guard<std::mutex> lock(ctx->mu);
-  const size_t rej_bytes = reject_bytes(ctx, L, count);
+  const size_t rej_bytes = reject_bytes(ctx, L, count, err_bytes + (size_t)C * per_ct, s);
   if ((st = ctx->ensure_ws(err_bytes + rej_bytes + (size_t)C * per_ct))) return st;
   int32_t* err = reinterpret_cast<int32_t*>(ctx->ws);
   uint8_t* rej = reinterpret_cast<uint8_t*>(ctx->ws) + err_bytes;
@@ -2873,13 +2899,20 @@ int shg_bfv_mul(shg_context* ctx, uint64_t* out, const uint64_t* a, const uint64
   const size_t want = ctx->chunk_cts > 0 ? (size_t)ctx->chunk_cts
                       : lanes.n > 1      ? std::min<size_t>(most, (count + 1) / 2)
                                          : most;
-  const int C = (int)std::min<size_t>((size_t)count, want);
-  const int nchunks = (count + C - 1) / C;
+  int C = (int)std::min<size_t>((size_t)count, want);
   // Never less than one lane's chunks of this batch: a smaller batch, or one on a
-  // single lane, then fits the scratch that a larger one left (a capture cannot grow it).
+  // single lane, then fits the scratch that a larger one left (a capture cannot grow
+  // it, and otherwise takes the lanes and chunks that it holds).
   const size_t alone = ctx->chunk_cts > 0 ? (size_t)ctx->chunk_cts
                                           : std::max<size_t>(1, ((size_t)1 << 30) / per_ct);
-  const size_t scratch_cts = std::max((size_t)lanes.n * C, std::min<size_t>(count, alone));
+  size_t scratch_cts = std::max((size_t)lanes.n * C, std::min<size_t>(count, alone));
+  if (!ctx->ws_fits(scratch_cts * per_ct, s)) {
+    const size_t room = ctx->ws_bytes / per_ct;
+    if (room < (size_t)lanes.n) lanes.n = 1;
+    C = std::max(1, (int)std::min<size_t>(C, room / lanes.n));
+    scratch_cts = (size_t)lanes.n * C;
+  }
+  const int nchunks = (count + C - 1) / C;
   if ((st = ctx->ensure_ws(scratch_cts * per_ct))) return st;
   if ((st = lanes.fork())) return st;
   for (int i = 0; i < nchunks; ++i) {
