@@ -410,7 +410,9 @@ int ks_chunk(const shg_context* ctx, size_t per_ct, int count, size_t budget, in
 // Streams that the independent parts of one batched call rotate over: lane 0 is
 // the caller's, the others the context's (made outside any stream capture, by
 // the first call that wants them; without them there is one lane).  Parts on
-// other lanes fill the tails of each other's launches.  Under ctx->mu.
+// other lanes fill the tails of each other's launches.  A capture holds the side
+// streams that its calls forked to until it ends: calls outside it go without
+// these lanes.  Under ctx->mu.
 struct KsLanes {
   shg_context* ctx;
   cudaStream_t s;
@@ -429,7 +431,20 @@ struct KsLanes {
       }
     }
     n = lanes_of(want);
+    for (int i = 0; i + 1 < n; ++i)
+      if (held_elsewhere(ctx->ks_side[i])) n = i + 1;
     return SHG_OK;
+  }
+  // Whether `side` is part of a capture that s is not.
+  bool held_elsewhere(cudaStream_t side) const {
+    cudaStreamCaptureStatus cap_side, cap_s;
+    unsigned long long id_side = 0, id_s = 0;
+    if (cudaStreamGetCaptureInfo(side, &cap_side, &id_side) == cudaSuccess &&
+        cap_side == cudaStreamCaptureStatusNone)
+      return false;
+    return cap_side != cudaStreamCaptureStatusActive ||
+           cudaStreamGetCaptureInfo(s, &cap_s, &id_s) != cudaSuccess ||
+           cap_s != cudaStreamCaptureStatusActive || id_s != id_side;
   }
   int lanes_of(int want) const {
     return ctx->ks_fork ? std::max(1, std::min(ctx->ks_lanes, want)) : 1;
