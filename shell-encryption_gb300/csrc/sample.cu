@@ -139,8 +139,8 @@ __host__ __device__ __forceinline__ int error_per_pass(int k2) {
 }
 
 // Error coefficients j0 .. j0 + J - 1 of one ciphertext into err: coefficient j
-// takes stream bytes [e0 + j * B, e0 + (j + 1) * B), kept in `bytes` (shared, at
-// least THREADS * 64) between their generation and the counting.
+// takes stream bytes [e0 + j * B, e0 + (j + 1) * B), kept in `bytes` (shared, aligned
+// to words, at least THREADS * 64) between their generation and the counting.
 template <int THREADS>
 __device__ __forceinline__ void error_pass(uint8_t* bytes, const uint32_t (&key)[8], uint64_t e0,
                                            int j0, int J, int k2, int32_t* err) {
@@ -343,7 +343,7 @@ __global__ void __launch_bounds__(kGuessThreads)
     k_sample_guess(uint64_t* a_dst, size_t a_stride, int negate, int32_t* err,
                    const uint8_t* seeds, int L, int variance, int log_n, int uniform_ctas,
                    Rejects* rejects, CtxDev c) {
-  __shared__ uint8_t bytes[kGuessThreads * 64];
+  __shared__ __align__(16) uint8_t bytes[kGuessThreads * 64];
   const int p = blockIdx.y, n = 1 << log_n;
   const unsigned total = (unsigned)L << log_n;
   uint32_t key[8];
@@ -382,7 +382,7 @@ __global__ void __launch_bounds__(kGuessThreads)
     k_sample_fix(uint64_t* a_dst, size_t a_stride, int negate, int32_t* err,
                  const uint8_t* seeds, int L, int variance, int log_n, int uniform_ctas,
                  Rejects* rejects, CtxDev c) {
-  __shared__ uint8_t bytes[kGuessThreads * 64];
+  __shared__ __align__(16) uint8_t bytes[kGuessThreads * 64];
   __shared__ Rejects rec;
   const int p = blockIdx.y, n = 1 << log_n;
   // Another CTA of this ciphertext may raise the count meanwhile; then what this
