@@ -55,7 +55,8 @@ int shg_profile_start(void);
 int shg_profile_stop(void);
 int shg_profile_query(const char* kernel, double* total_ms, uint64_t* launches);
 /* Reserve scratch space for batched calls up front (so a later call can be
- * captured into a graph without allocating). */
+ * captured into a graph without allocating; a captured call makes do with less
+ * than it would take otherwise). */
 int shg_context_reserve(shg_context* ctx, size_t bytes);
 /* Ciphertexts per internal chunk of the batched key-switch pipeline
  * (0 = default). */
@@ -84,7 +85,10 @@ int shg_debug_status(unsigned* first_failure);
  * queries of an oblivious expansion rotate over, 1 to 4 (2 =
  * default: the caller's stream and a second one, so one chunk fills the
  * other's tail; 1 = the caller's stream only, e.g. to time kernels one at a
- * time).  Each lane holds its own chunk of digit scratch. */
+ * time).  BFV products of eight pairs and more take two of them, or one at 1.
+ * Each lane holds its own chunk of scratch; a captured call uses as many lanes
+ * as the scratch that is there holds, and a call beside a capture of the same
+ * context none that the capture holds. */
 int shg_context_set_ks_lanes(shg_context* ctx, int lanes);
 /* shg_bgv_mul_relin_host pipeline shape: ciphertexts per piece (default 32)
  * and device staging slots in flight (default 4, at most 8). */

@@ -1226,10 +1226,13 @@ void make_form32(shg_context* ctx, const shg_key* key) {
 // The key's 32-bit form if a key switch of `count` ciphertexts with this one
 // key should use it (ks32.cu), else an empty one.  Counted in 64-bit transforms
 // of n, it saves k L of them and costs 0.45 of one per 32-bit transform (3 k + 6 L)
-// and 2 L; two more launches need a saving of about 1.75 M coefficients (measured
-// break-even: n = 2^14, 6 limbs between 1 and 2 ciphertexts (49.7 / 53.6 and
-// 69.8 / 63.7 us), 4 limbs at 6 (83.3 / 84.0); n = 2^13, 4 limbs between 8 and 16
-// (61.7 / 65.5 and 97.6 / 92.4); n = 2^12, 12 limbs at 2 (71.6 / 74.1)).
+// and 2 L, beside two more launches.  Products through the rows and through the
+// form, us, by the coefficients saved: n = 2^14, six limbs, 1 ciphertext 41.1 / 40.4
+// (0.91 M), 2 58.7 / 50.6 (1.82 M); four limbs, 4 53.4 / 53.5 (0.85 M), 8 90.6 / 77.4
+// (1.70 M); n = 2^13, six limbs, 2 39.0 / 40.4 (0.91 M), 4 55.4 / 50.0 (1.82 M);
+// n = 2^12, twelve limbs, 1 45.2 / 48.3 (1.34 M), 2 60.4 / 56.3 (2.68 M).  They meet
+// between 0.9 and 1.4 M; the line at 1.75 M leaves the form's memory alone where it
+// gains less than a fifth.
 //
 // `make`: the call may make the words; a capture of s takes them only if they are
 // there.  Keys that only multi-key batches use thus never hold them.  Under ctx->mu.
@@ -1428,8 +1431,8 @@ int keyswitch(shg_context* ctx, const shg_key* key, uint64_t* out,
   const size_t Ln = (size_t)L * n;
   const size_t tab_bytes = keys ? 2 * (size_t)count * sizeof(void*) : 0;
   std::lock_guard<std::mutex> lock(ctx->mu);
-  // Each lane has its own X and D; two chunks side by side take three quarters of
-  // the time (250 rotations at n = 2^14, six limbs: 2971 -> 2268 us).
+  // Each lane has its own X and D; two chunks side by side take 18 % less time (250
+  // rotations at n = 2^14, six limbs: 2215 us, 2703 on one lane).
   KsLanes lanes{ctx, s};
   KsPlan p;
   int st = plan_ks(lanes, key, count, keys == nullptr, Ln * sizeof(uint64_t), tab_bytes,
@@ -2036,7 +2039,7 @@ int run_expand(shg_context* ctx, const shg_key* const* keys, int levels, uint64_
   // Queries are independent: each lane takes its share of them through all
   // levels with its own X, D and KS, so one lane's memory-bound level update
   // runs beside another's digit transforms (24 queries of 10 levels at
-  // n = 2^12: 12.8 -> 11.3 ms).
+  // n = 2^12: 10.2 ms against 11.0 on one lane).
   KsLanes lanes{ctx, s, plan.lanes};
   const CtxDev dv = ctx->dev();
   int st = lanes.fork();

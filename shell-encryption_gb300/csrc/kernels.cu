@@ -634,7 +634,11 @@ __global__ void k_expand_combine(uint64_t* base, const uint64_t* ks,
 // kExpandTile >= 2^(j + 1) positions of one member and reads every base value
 // before it writes one.  Two pairs of positions per thread keep six 16-byte loads in flight.
 // 512 members at n = 2^12, k = 8: 64 us against 56 + 22 as two kernels (the
-// key-switched member went through memory between them).
+// key-switched member went through memory between them), all on transforms of one
+// CTA per limb.  It runs where those do: n = 2^10 and 2^11, or higher rings with the
+// four-step threshold raised; n = 2^12 takes the four-step key switch and
+// k_expand_combine by default, which together are faster (24 queries of 10 levels
+// 10.2 ms against 11.3).
 constexpr int kExpandTile = 1024;
 __global__ void __launch_bounds__(256, 3)
     k_ks_expand(uint64_t* base, const uint64_t* D, const uint64_t* kb, const uint64_t* ka, int k,
@@ -1336,7 +1340,7 @@ void launch_expand_combine(const CtxDev& c, uint64_t* base, const uint64_t* ks,
                                                         half, total, c.log_n, c);
 }
 
-// Grid of the word kernels: (limb, tile) by polynomials, about 16 CTAs per SM.
+// Grid of the word kernels: (limb, tile) by polynomials, about 32 CTAs per SM.
 static dim3 ser_grid(const CtxDev& c, int count, int L) {
   const int x = L * (c.log_n > 10 ? 1 << (c.log_n - 10) : 1);
   return dim3(x, std::max(1, std::min(count, std::min(65535, c.sms * 32 / x + 1))));

@@ -173,8 +173,8 @@ __device__ __forceinline__ void after_previous() {
 // this library went onto the stream just before, no event wait or copy) its CTAs
 // are placed once the last CTA before it has exited, without the drain and
 // launch between two kernels, about 2 us: at n = 2^14, six 45-bit primes, one
-// ct-mult+relin 48 -> 41 us, two 64 -> 51, two inverse NTTs 14.5 -> 12.4, four forward
-// 16.6 -> 12.6, one BFV product 146 -> 105; batches that fill the GPU for many waves are within 1 %.  No kernel
+// ct-mult+relin 47.4 -> 41.0 us, two 62.2 -> 50.0, two inverse NTTs 14.4 -> 12.3, four
+// forward 15.5 -> 12.4, one BFV product 142 -> 104; batches that fill the GPU for many waves are within 1 %.  No kernel
 // triggers its successor itself: at its start, the waiting CTAs crowd onto the SMs
 // that have room (two inverse NTTs 18.5 us) and hold slots that another lane
 // would use (250 rotations 2230 -> 2315 us); before its stores, k32_rows loses

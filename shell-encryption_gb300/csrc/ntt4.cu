@@ -872,11 +872,12 @@ __global__ void __launch_bounds__(32 * W, MB)
 // (blockIdx.y: the class; they read the same twiddles), else four rows of one
 // transform (no idle rows in small batches, four times the twiddles).
 //
-// Bound by the multiply pipe and the latency of its loads; 25 instructions per
-// butterfly where the kernels before it took 33 and more (four two-level passes
-// with three exchanges, or CTA-wide barriers).  n = 2^14, six 45-bit primes: 512
-// polynomials 429 -> 420 us, ModReduce of 256 308 -> 290, the transforms of 200
-// encryptions 278 -> 268.
+// Bound by the multiply pipe (67 % busy) and the latency of its loads (4.4 warps
+// waiting for them per issued instruction); 26 instructions per butterfly where the
+// warp-per-row form takes 31 (four two-level passes with three exchanges) and the
+// CTA-per-row form has barriers.  n = 2^14, six 45-bit primes: 512 polynomials
+// 429 -> 423 us, ModReduce of 256 308 -> 289, the transforms of 200 encryptions
+// 278 -> 268.
 struct RowTile64 {
   static constexpr int kStride = 152;  // words of a row
   uint64_t* sm;                        // the warp's four rows
