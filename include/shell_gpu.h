@@ -182,9 +182,8 @@ int shg_ct_tensor(shg_context* ctx, uint64_t* out, const uint64_t* a,
  * Keys of at least four limbs at n = 2^12 .. 2^15 with primes below 2^57 and at
  * most 128 digits of at most 26 bits, all below every prime, have a 32-bit form
  * beside the rows: 1.5 times their size.  The first batch with this one key that
- * is large enough to gain from it makes the form (with another 1.25 times the
- * rows for the time of the making) while a quarter of the device's memory stays
- * free; batches with one key per member, captures and shg_relin_apply_noalloc
+ * is large enough to gain from it makes the form, while a quarter of the
+ * device's memory stays free; batches with one key per member, captures and shg_relin_apply_noalloc
  * never make it.  It goes back when an allocation of this library finds the
  * device full, but not once a captured call has used it.  Results are the same
  * with and without. */

@@ -388,7 +388,7 @@ namespace {
 // Workspaces hold the larger need of the two, so that a call of fewer
 // ciphertexts (which may take the other form) never needs more than one of more.
 size_t ks_scratch_bytes(const shg_context* ctx, const shg_key* key, const shg::Ks32& ks32) {
-  if (ks32.key) return shg::ks32_scratch_bytes(key->k, key->L) * ctx->n;
+  if (ks32.crt) return shg::ks32_scratch_bytes(key->k, key->L) * ctx->n;
   return (size_t)key->k * key->L * ctx->n * sizeof(uint64_t);
 }
 
@@ -1168,59 +1168,55 @@ void plan_form32(shg_context* ctx, shg_key* key, const std::vector<DigitDesc>& d
   key->bytes += f.bytes;
 }
 
-// Makes the words of the key's form (under ctx->mu; the calling stream is not
-// being captured) while a quarter of the device's memory stays free, else leaves
-// the key to its rows and looks again 256 calls later.  On a stream of its own and
-// in relaxed capture mode, so that a capture of another stream is not disturbed.
-// 0.57 ms for six limbs at n = 2^14 (42 MB beside 28 MB of rows), 2.1 ms for twelve
+// Makes the words of the key's form while a quarter of the device's memory stays
+// free, else leaves the key to its rows for 256 calls.  Under ctx->mu, on the
+// stream of a call that is not being captured, in the scratch made ready for it, as
+// many digits at a time as that holds; in relaxed capture mode, so that a capture of
+// another stream is not disturbed.  True once they are there for any stream.
+// 0.4 ms for six limbs at n = 2^14 (42 MB beside 28 MB of rows), 1.9 ms for twelve
 // at n = 2^15 (340 beside 226 MB), once per key.
-void make_form32(shg_context* ctx, const shg_key* key) {
+bool make_form32(shg_context* ctx, const shg_key* key, cudaStream_t s) {
   shg_key::Form32& f = key->form32;
-  if (f.wait > 0) {
-    --f.wait;
-    return;
-  }
-  f.wait = 256;
   const int L = key->L, k = key->k;
-  const size_t elems = (size_t)k * L * ctx->n;
-  const size_t row_bytes = elems * sizeof(uint64_t), tmp_bytes = 3 * elems * sizeof(uint32_t);
+  const size_t Ln = (size_t)L * ctx->n;
+  const size_t digit_bytes = Ln * (sizeof(uint64_t) + 3 * sizeof(uint32_t));
+  const int per = (int)std::min<size_t>(k, ctx->ws_bytes / digit_bytes);
+  f.wait = 256;
+  if (per == 0) return false;
   cudaStreamCaptureMode mode = cudaStreamCaptureModeRelaxed;
   cudaThreadExchangeStreamCaptureMode(&mode);
-  uint64_t* rows = nullptr;
-  uint32_t *tmp = nullptr, *words = nullptr;
-  cudaStream_t s = nullptr;
+  uint64_t* rows = ctx->ws;
+  uint32_t* tmp = reinterpret_cast<uint32_t*>(rows + per * Ln);
+  uint32_t* words = nullptr;
   size_t room = 0, total = 0;
   cudaError_t e = cudaMemGetInfo(&room, &total);
-  if (e == cudaSuccess && room < f.bytes + row_bytes + tmp_bytes + total / 4)
-    e = cudaErrorMemoryAllocation;
-  if (e == cudaSuccess) e = cudaStreamCreateWithFlags(&s, cudaStreamNonBlocking);
-  if (e == cudaSuccess) e = cudaMalloc(&rows, row_bytes);
-  if (e == cudaSuccess) e = cudaMalloc(&tmp, tmp_bytes);
+  if (e == cudaSuccess && room < f.bytes + total / 4) e = cudaErrorMemoryAllocation;
   if (e == cudaSuccess) e = cudaMalloc(&words, f.bytes);
   if (e == cudaSuccess) {
     for (int c = 0; c < 2; ++c) {
-      // the stored rows carry 2^64 mod q: the export scaling takes it off
-      shg::launch_ntt_inv(ctx->dev(), c ? key->ka : key->kb, rows, k * L, L, 1, s);
-      shg::launch_ks32_key(ctx->dev(), f.ks.w, rows, tmp, k, L, c, words, s);
+      for (int j = 0; j < k; j += per) {
+        const int nj = std::min(per, k - j);
+        // the stored rows carry 2^64 mod q: the export scaling takes it off
+        shg::launch_ntt_inv(ctx->dev(), (c ? key->ka : key->kb) + j * Ln, rows, nj * L, L, 1, s);
+        shg::launch_ks32_key(ctx->dev(), f.ks.w, rows, tmp, j, nj, k, L, c, words, s);
+      }
     }
     e = cudaGetLastError();
     const cudaError_t done = cudaStreamSynchronize(s);
     if (e == cudaSuccess) e = done;
   }
-  cudaFree(rows);
-  cudaFree(tmp);
-  if (s) cudaStreamDestroy(s);
-  if (e == cudaSuccess) {
-    f.words = words;
-    f.ks.key = words;
-    f.wait = 0;
-    std::lock_guard<std::mutex> list(g_forms_mu);
-    g_forms.push_back(key);
-  } else {
+  cudaThreadExchangeStreamCaptureMode(&mode);
+  if (e != cudaSuccess) {
     cudaGetLastError();
     cudaFree(words);
+    return false;
   }
-  cudaThreadExchangeStreamCaptureMode(&mode);
+  f.words = words;
+  f.ks.key = words;
+  f.wait = 0;
+  std::lock_guard<std::mutex> list(g_forms_mu);
+  g_forms.push_back(key);
+  return true;
 }
 
 // The key's 32-bit form if a key switch of `count` ciphertexts with this one
@@ -1234,10 +1230,11 @@ void make_form32(shg_context* ctx, const shg_key* key) {
 // between 0.9 and 1.4 M; the line at 1.75 M leaves the form's memory alone where it
 // gains less than a fifth.
 //
-// `make`: the call may make the words; a capture of s takes them only if they are
-// there.  Keys that only multi-key batches use thus never hold them.  Under ctx->mu.
+// `make`: the call can make the words where the form has none yet (ks.key is
+// nullptr); a capture of s takes them only if they are there.  Keys that only
+// multi-key batches use thus never hold them.  Under ctx->mu.
 const shg::Ks32& ks32_for(shg_context* ctx, const shg_key* key, int count, bool one_key,
-                          cudaStream_t s, bool make = true) {
+                          cudaStream_t s, bool make) {
   static const shg::Ks32 none;
   const CtxDev c = ctx->dev();
   shg_key::Form32& f = key->form32;
@@ -1249,12 +1246,16 @@ const shg::Ks32& ks32_for(shg_context* ctx, const shg_key* key, int count, bool 
   cudaStreamCaptureStatus cap = cudaStreamCaptureStatusNone;
   const bool captured = cudaStreamIsCapturing(s, &cap) != cudaSuccess ||
                         cap != cudaStreamCaptureStatusNone;
-  if (!f.words && make && !captured) make_form32(ctx, key);
-  if (!f.words) return none;
+  if (!f.words) {
+    if (!make || captured) return none;
+    if (f.wait > 0) {
+      --f.wait;
+      return none;
+    }
+  }
   f.captured |= captured;
   return f.ks;
 }
-
 
 }  // namespace
 
@@ -1405,7 +1406,7 @@ int plan_ks(KsLanes& lanes, const shg_key* key, int count, bool one_key, size_t 
     p->ks32 = &ks32_for(ctx, key, count, one_key, lanes.s, make);
     p->per_ct = x_per_ct + ks_scratch_bytes(ctx, key, *p->ks32);
     p->C = ks_chunk(ctx, p->per_ct, count, budget, set_max);
-    const bool form = p->ks32->key != nullptr;
+    const bool form = p->ks32->crt != nullptr;
     int st = lanes.open((count + p->C - 1) / p->C);
     if (st) return st;
     size_t need = std::max(
@@ -1417,8 +1418,8 @@ int plan_ks(KsLanes& lanes, const shg_key* key, int count, bool one_key, size_t 
       need = lanes.n * p->per_ct * p->C;
     }
     if ((st = ctx->ensure_ws(need + fixed))) return st;
-    // the workspace may have taken the form's memory: `need` holds the other layout
-    if (!form || p->ks32->key) return SHG_OK;
+    // no room for the form, or the workspace took its memory: `need` holds the other layout
+    if (!form || p->ks32->key || (make && make_form32(ctx, key, lanes.s))) return SHG_OK;
   }
 }
 
@@ -1652,10 +1653,10 @@ int mul_relin_host_impl(shg_context* ctx, const shg_key* key, void* out_v, const
     ks32 = &ks32_for(ctx, key, count, true, (cudaStream_t)stream, make);
     d_per_ct = ks_scratch_bytes(ctx, key, *ks32);
     C = chunk_of(d_per_ct);
-    form = ks32->key != nullptr;
+    form = ks32->crt != nullptr;
     if ((st = ctx->ensure_ws(lanes * std::max(C * d_per_ct, chunk_of(d_plain) * d_plain))))
       return st;
-    if (ks32->key) break;
+    if (ks32->key || (form && make && make_form32(ctx, key, (cudaStream_t)stream))) break;
   }
   uint64_t* D0 = ctx->ws;
   for (cudaStream_t& s : ctx->io_streams)

@@ -305,10 +305,10 @@ void launch_ks32(const CtxDev& c, const Ks32& ks, uint64_t* scratch, const uint6
                  const DigitDesc* digits, int k, uint64_t* out, const uint64_t* base,
                  size_t base_ct_elems, CtMap map, int base1_zero, int subst_power, int count,
                  int L, cudaStream_t s);
-// Imports component `comp` of a key: rows [k][L][n] in coefficient form, tmp
-// [k][L][3][n] scratch.
-void launch_ks32_key(const CtxDev& c, const W32& w, const uint64_t* rows, uint32_t* tmp, int k,
-                     int L, int comp, uint32_t* key, cudaStream_t s);
+// Imports digits j .. j + nj - 1 of component `comp` of a key of k: rows [nj][L][n] in
+// coefficient form, tmp [nj][L][3][n] scratch.
+void launch_ks32_key(const CtxDev& c, const W32& w, const uint64_t* rows, uint32_t* tmp, int j,
+                     int nj, int k, int L, int comp, uint32_t* key, cudaStream_t s);
 // Row phase of the forward transforms buf [count][2][L][n] (column phase done)
 // plus the key switch's base: out [count][2][L][n].
 void launch4_rows_add(const CtxDev& c, const uint64_t* buf, uint64_t* out, const uint64_t* base,

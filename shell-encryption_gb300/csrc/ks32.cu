@@ -334,12 +334,12 @@ __global__ void __launch_bounds__(K32<LOG_N>::THREADS)
   }
 }
 
-// Key import, row phase: the CTA takes one row of every digit and limb of one
-// prime and writes them, times `scale`, to their places in the key of
-// k32_rows (component comp).
+// Key import, row phase: the CTA takes one row of digits j .. j + nj - 1 and every
+// limb of one prime and writes them, times `scale`, to their places in the key of
+// k32_rows (k digits, component comp).
 template <int LOG_N>
 __global__ void __launch_bounds__(128)
-    k32_key_rows(const uint32_t* in, int k, int L, int comp, uint32_t* key,
+    k32_key_rows(const uint32_t* in, int j, int nj, int k, int L, int comp, uint32_t* key,
                  const __grid_constant__ W32 w) {
   __shared__ __align__(16) uint32_t sm[16 * kRow32];
   __shared__ __align__(16) uint2 tw[kRowTw32];
@@ -351,9 +351,9 @@ __global__ void __launch_bounds__(128)
       row_tw_fwd(w.fwd + ((size_t)a << LOG_N), R, row, threadIdx.x);
   __syncthreads();
   uint32_t* tile = sm + warp * 4 * kRow32;
-  for (int q0 = warp * 4; q0 < k * L; q0 += 16) {
+  for (int q0 = warp * 4; q0 < nj * L; q0 += 16) {
     for (int i = lane; i < 512; i += 32) {
-      const size_t jl = min(q0 + (i >> 7), k * L - 1);
+      const size_t jl = min(q0 + (i >> 7), nj * L - 1);
       tile[(i >> 7) * kRow32 + row_word32(i & 127)] =
           in[((jl * 3 + a) << LOG_N) + row * 128 + (i & 127)];
     }
@@ -364,8 +364,8 @@ __global__ void __launch_bounds__(128)
     __syncwarp();
     for (int i = lane; i < 512; i += 32) {
       const int jl = q0 + (i >> 7);
-      if (jl < k * L)
-        key[((size_t)blockIdx.x * k * L + jl) * 256 + comp * 128 + (i & 127)] =
+      if (jl < nj * L)
+        key[(((size_t)blockIdx.x * k + j) * L + jl) * 256 + comp * 128 + (i & 127)] =
             tile[(i >> 7) * kRow32 + row_word32(i & 127)];
     }
     __syncwarp();
@@ -470,14 +470,14 @@ void launch_ks32(const CtxDev& c, const Ks32& ks, uint64_t* scratch, const uint6
   launch4_rows_add(c, Y, out, base, base_ct_elems, map, base1_zero, subst_power, count, L, s);
 }
 
-void launch_ks32_key(const CtxDev& c, const W32& w, const uint64_t* rows, uint32_t* tmp, int k,
-                     int L, int comp, uint32_t* key, cudaStream_t s) {
+void launch_ks32_key(const CtxDev& c, const W32& w, const uint64_t* rows, uint32_t* tmp, int j,
+                     int nj, int k, int L, int comp, uint32_t* key, cudaStream_t s) {
   LaunchScope scope_("ks32_key", s);
   g_launch_count++;  // second phase kernel
 #define F(LN)                                                                          \
   {                                                                                    \
-    k32_key_cols<LN><<<k * L * K32<LN>::TILES, K32<LN>::THREADS, 0, s>>>(rows, L, tmp, w, c); \
-    k32_key_rows<LN><<<3 * (1 << (LN - 7)), 128, 0, s>>>(tmp, k, L, comp, key, w); \
+    k32_key_cols<LN><<<nj * L * K32<LN>::TILES, K32<LN>::THREADS, 0, s>>>(rows, L, tmp, w, c); \
+    k32_key_rows<LN><<<3 * (1 << (LN - 7)), 128, 0, s>>>(tmp, j, nj, k, L, comp, key, w); \
   }
   SHG_DISPATCH32(c.log_n, F)
 #undef F
